@@ -4,6 +4,7 @@
 
 #include "api_error.hpp"
 
+#include "chan_fused.hpp"
 #include "chan_plain.cuh"
 #include "chan_tc.cuh"
 #include "chan_wide.cuh"
@@ -177,6 +178,8 @@ struct rfx_chan_plan {
     void* twiddles;       // tensor core: the DFT operand image, built once in FP64
     void* scratch;        // plain: channel outputs before their magnitude (first such call);
                           // tensor core, 1024 channels: the branch sums (made with the plan)
+    bool fused;           // RFX_CHAN_AUTO at 64 channels: the fused FP32 kernel, within the
+                          // limits of the tensor-core form's plans
 };
 
 extern "C" {
@@ -515,8 +518,9 @@ int rfx_chan_plan_create(int impl, int channels, int64_t max_samples, rfx_chan_p
         return fail(RFX_ERR_INVALID, "channelize: null plan pointer");
     }
     *plan = nullptr;
+    bool fused = false;
     if (impl == RFX_CHAN_AUTO) {
-        impl = rfx::tuned_chan_impl(channels, max_samples);
+        impl = rfx::tuned_chan_impl(channels, max_samples, &fused);
     }
     if (impl != RFX_CHAN_PLAIN && impl != RFX_CHAN_TC) {
         return fail(RFX_ERR_INVALID, "channelize: unknown implementation %d", impl);
@@ -529,7 +533,11 @@ int rfx_chan_plan_create(int impl, int channels, int64_t max_samples, rfx_chan_p
                     static_cast<long long>(max_samples), static_cast<long long>(kMaxSamples));
     }
     auto* p = new rfx_chan_plan{impl, channels, rfx_channelize_frames(max_samples, channels), 0,
-                                false, nullptr, nullptr};
+                                false, nullptr, nullptr, fused};
+    if (fused) {
+        *plan = p;   // its one kernel needs nothing beside the call's arguments
+        return RFX_OK;
+    }
     if (impl == RFX_CHAN_TC) {
         const bool wide = rfx::chan_wide_supported(channels);
         if (!wide && !rfx::chan_tc_supported(channels, 1)) {
@@ -692,6 +700,14 @@ int channelize_plan(rfx_chan_plan* plan, const void* x, const float* taps, void*
                                           "shared memory",
                         num_taps);
         }
+        if (plan->fused) {
+            if (num_samples < plan->channels) {
+                return cuda_fail(cudaErrorInvalidValue, "chan_fused_launch");
+            }
+            const cudaError_t err = rfx::chan_fused_launch(
+                x, taps, out, frames, plan->channels, num_taps, magnitude, format, stream);
+            return err == cudaSuccess ? RFX_OK : cuda_fail(err, "chan_fused_launch");
+        }
         const cudaError_t err = rfx::chan_tc_launch(x, taps, plan->twiddles, out, num_samples,
                                                     num_taps, stream, magnitude, format);
         return err == cudaSuccess ? RFX_OK : cuda_fail(err, "chan_tc_launch");
@@ -699,6 +715,11 @@ int channelize_plan(rfx_chan_plan* plan, const void* x, const float* taps, void*
     if (frames != plan->frames) {
         return fail(RFX_ERR_INVALID, "channelize: plan made for %lld frames, call has %lld",
                     static_cast<long long>(plan->frames), static_cast<long long>(frames));
+    }
+    if (rfx::chan_fused_supported(plan->channels, num_taps)) {
+        const cudaError_t err = rfx::chan_fused_launch(x, taps, out, frames, plan->channels,
+                                                       num_taps, magnitude, format, stream);
+        return err == cudaSuccess ? RFX_OK : cuda_fail(err, "chan_fused_launch");
     }
     void* z = out;
     if (magnitude) {

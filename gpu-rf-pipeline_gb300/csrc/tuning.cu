@@ -301,16 +301,18 @@ TcConfig tuned_fir_tc_config(int num_taps, long long n)
     return fir_tcw_supported(num_taps) ? TcConfig{kTcWindowTile, 4} : TcConfig{96, 6};
 }
 
-// Built-in rule: the fused tensor-core form at 64 channels (one HBM pass against the plain
-// form's two); cuFFT's plain form elsewhere, including 1024 channels, where the branch-sum
-// kernel + cuFFT measured faster than the factored tensor-core DFT on GB300.
-int tuned_chan_impl(int channels, long long n)
+// Built-in rule: at 64 channels the fused FP32 kernel (chan_fused.cuh) where the tensor-core form
+// stood; the plain form elsewhere, including 1024 channels, where the branch-sum kernel + cuFFT
+// measured faster than the factored tensor-core DFT on GB300.
+int tuned_chan_impl(int channels, long long n, bool* fused)
 {
     ChanEntry e;
+    *fused = false;
     if (lookup_chan(channels, n, &e)) {
         return e.impl;
     }
-    return chan_tc_supported(channels, 1) ? RFX_CHAN_TC : RFX_CHAN_PLAIN;
+    *fused = chan_tc_supported(channels, 1);
+    return *fused ? RFX_CHAN_TC : RFX_CHAN_PLAIN;
 }
 
 }  // namespace rfx

@@ -59,15 +59,19 @@ typedef enum rfx_fir_impl {
 
 /* Channelizer implementations. */
 typedef enum rfx_chan_impl {
-    /* FP32 branch-sum kernel (bit-identical to the project's channelize_branch_kernel) followed
-     * by cuFFT's batched in-place inverse transform, as the project computes it. */
+    /* FP32 branch sums (bit-identical to the project's channelize_branch_kernel) and the inverse
+     * transform in FP32: one fused kernel for 16, 32, ..., 512 channels and at most 32 taps per
+     * branch; otherwise a branch-sum kernel followed by cuFFT's batched in-place inverse
+     * transform, as the project computes it. */
     RFX_CHAN_PLAIN = 0,
     /* The M-point DFT as a split-FP16 complex GEMM on tcgen05. M = 64: one fused kernel (FP32
      * branch sums into shared memory, then the GEMM). M = 1024: the plain form's FP32 branch
      * sums, then the DFT factored 32 x 32 into two GEMMs with an FP32 twiddle between them. */
     RFX_CHAN_TC = 1,
     /* Chosen when the plan is made, from the tuned table (rfx_autotune_channelize) or the
-     * built-in rule (the tensor-core form at 64 channels, the plain form otherwise). */
+     * built-in rule: the plain form, whose fused kernel at 64 channels runs in plans that take
+     * what the tensor-core form's take (any call up to the plan's length, at least one whole
+     * frame, at most 2048 taps). */
     RFX_CHAN_AUTO = 2
 } rfx_chan_impl;
 
@@ -198,8 +202,8 @@ typedef struct rfx_chan_plan rfx_chan_plan;
  * RFX_CHAN_PLAIN, the batched inverse cuFFT plan of `channels` points (the project's FftPlan,
  * src/fft_plan.hpp:15-22); for RFX_CHAN_TC (64 or 1024 channels, RFX_ERR_CAPACITY otherwise),
  * the DFT operand built in FP64 and, at 1024 channels, a buffer for the branch sums
- * (max_samples / 1024 frames x 8 KB). RFX_CHAN_AUTO picks by the tuned table, else the
- * tensor-core form at 64 channels.
+ * (max_samples / 1024 frames x 8 KB). RFX_CHAN_AUTO picks by the tuned table, else the fused
+ * FP32 kernel at 64 channels and the plain form otherwise.
  * Allocates; call outside timed regions. */
 int rfx_chan_plan_create(int impl, int channels, int64_t max_samples, rfx_chan_plan** plan);
 int rfx_chan_plan_destroy(rfx_chan_plan* plan);
@@ -219,9 +223,9 @@ int rfx_channelize_branches(const void* x, const float* taps, void* u, int64_t n
 
 /* The channelizer followed by the magnitude of every channel output, mag[t][k] = |z[t][k]|
  * (frames x channels float32). Tensor-core plans compute it in the DFT-GEMM epilogue, so the
- * complex channel outputs never reach HBM; plain plans run the magnitude kernel over the
- * channel outputs in a plan-owned buffer (allocated by the first such call). mag 16-byte
- * aligned. Fuses channelize |> magnitude (compiler/examples/channelizer.sf,
+ * complex channel outputs never reach HBM, and so does the plain form's fused kernel; other
+ * plain plans run the magnitude kernel over the channel outputs in a plan-owned buffer (allocated
+ * by the first such call). mag 16-byte aligned. Fuses channelize |> magnitude (compiler/examples/channelizer.sf,
  * src/magnitude.cu:17-25); no single-call counterpart in the project. */
 int rfx_channelize_magnitude_launch(rfx_chan_plan* plan, const void* x, const float* taps,
                                     float* mag, int64_t num_samples, int num_taps,
@@ -347,7 +351,7 @@ int rfx_magnitude_host(const void* x_iq, int64_t num_samples, float* mag, rfx_be
 
 /* The `auto` implementations consult in-process tables filled by the calls below, and apply
  * a built-in rule where an entry is missing (FIR: the tensor core from 32 taps and 2^16
- * samples; channelizer: the tensor core at 64 channels). A batch plan's auto form puts every
+ * samples; channelizer: the plain form). A batch plan's auto form puts every
  * capture of 2 taps or more on a tensor-core phase; rfx_fir_batch_launch's auto form follows
  * the FIR table beyond 385 taps and takes the tensor core from 160 taps (and 2^16 samples)
  * otherwise. If the environment variable RFX_TUNE_FILE names a file saved by
