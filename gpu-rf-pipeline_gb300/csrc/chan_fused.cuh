@@ -26,6 +26,7 @@
 // of the transform already keep the load/store pipe half busy.
 #pragma once
 
+#include "launch.hpp"
 #include "magnitude.cuh"
 #include "ptx.cuh"
 #include "sample_fmt.cuh"
@@ -373,6 +374,8 @@ chan_fused_kernel(const void* __restrict__ x, const float* __restrict__ taps,
     constexpr int r0 = Radices<M>::r[0];
     constexpr int r1 = Radices<M>::r[1];
     constexpr int r2 = Radices<M>::r[2];
+    wait_for_stream();
+    allow_next();
     // This branch's taps: in registers, or column m of taps_s[p][m].
     const int my_taps = m < num_taps ? (num_taps - m + M - 1) / M : 0;
     const int first_valid = m > 0 ? 1 : 0;   // x[dM - m] lies in the input from this d on
@@ -574,14 +577,6 @@ cudaError_t launch(const void* x, const float* taps, void* out, long long frames
             cudaSuccess) {
         return err;
     }
-    auto kernel = chan_fused_kernel<M, PG, kFmt, kMag>;
-    if (C::kBytes > 48u * 1024u) {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(C::kBytes));
-        if (err != cudaSuccess) {
-            return err;
-        }
-    }
     const long long groups = static_cast<long long>(sms) * C::kBlocks * C::kGroups;
     long long seg = (frames + groups - 1) / groups;
     seg = (seg + kR - 1) / kR * kR;
@@ -589,10 +584,18 @@ cudaError_t launch(const void* x, const float* taps, void* out, long long frames
     const unsigned blocks = static_cast<unsigned>((segs + C::kGroups - 1) / C::kGroups);
     const long long n = (frames - 1) * M + 1;
     const int guard = kR * (PG + 1);
-    kernel<<<blocks, C::kThreads, C::kBytes, stream>>>(x, taps, out, n, static_cast<int>(frames),
-                                                       num_taps, static_cast<int>(seg), guard,
-                                                       num_taps == kR * PG * M ? 1 : 0);
-    return cudaGetLastError();
+    const size_t bytes = even_spread_smem(C::kBytes, blocks, sms, C::kBlocks);
+    auto kernel = chan_fused_kernel<M, PG, kFmt, kMag>;
+    if (bytes > 48u * 1024u) {
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(bytes));
+        if (err != cudaSuccess) {
+            return err;
+        }
+    }
+    return launch_overlapped(kernel, blocks, C::kThreads, bytes, stream, x, taps, out, n,
+                             static_cast<int>(frames), num_taps, static_cast<int>(seg), guard,
+                             num_taps == kR * PG * M ? 1 : 0);
 }
 
 template <int M, int PG>

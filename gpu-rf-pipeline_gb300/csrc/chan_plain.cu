@@ -22,6 +22,7 @@
 // Frame groups whose terms fall before the input, and the last group (past its end), take a
 // path that tests every term.
 #include "chan_plain.cuh"
+#include "launch.hpp"
 #include "ptx.cuh"
 
 #include <cuda_runtime.h>
@@ -139,6 +140,8 @@ chan_branch_kernel(const void* __restrict__ x, const float* __restrict__ taps,
                    int num_taps, int width, int guard_frames)
 {
     extern __shared__ float taps_s[];   // [p][j]: tap p of branch blockIdx.y * width + j
+    wait_for_stream();
+    allow_next();
     const int j = static_cast<int>(threadIdx.x) % width;
     const int m = static_cast<int>(blockIdx.y) * width + j;
     if (kSmemTaps) {
@@ -226,6 +229,8 @@ chan_branch_ring_kernel(const void* __restrict__ x, const float* __restrict__ ta
     constexpr int kSb = kFmt == 0 ? 8 : 4;       // bytes per stored sample
     constexpr uint32_t kStageBytes = kR * kRingThreads * kSb;
     __shared__ __align__(16) unsigned char stage[kRingStages * kStageBytes];
+    wait_for_stream();
+    allow_next();
     const int tid = static_cast<int>(threadIdx.x);
     const int j = tid % width;
     const int m = static_cast<int>(blockIdx.y) * width + j;
@@ -371,16 +376,17 @@ static cudaError_t ring_launch(const void* x, const float* taps, float2* u, long
                                long long frames, int channels, int per_branch,
                                cudaStream_t stream, int format)
 {
-    const void* fn = nullptr;
+    void (*fn)(const void*, const float*, float2*, long long, long long, int, int, long long, int) =
+        nullptr;
     switch (per_branch / kR * 2 + format) {
-    case 2: fn = reinterpret_cast<const void*>(chan_branch_ring_kernel<1, 0>); break;
-    case 3: fn = reinterpret_cast<const void*>(chan_branch_ring_kernel<1, 1>); break;
-    case 4: fn = reinterpret_cast<const void*>(chan_branch_ring_kernel<2, 0>); break;
-    case 5: fn = reinterpret_cast<const void*>(chan_branch_ring_kernel<2, 1>); break;
-    case 6: fn = reinterpret_cast<const void*>(chan_branch_ring_kernel<3, 0>); break;
-    case 7: fn = reinterpret_cast<const void*>(chan_branch_ring_kernel<3, 1>); break;
-    case 8: fn = reinterpret_cast<const void*>(chan_branch_ring_kernel<4, 0>); break;
-    case 9: fn = reinterpret_cast<const void*>(chan_branch_ring_kernel<4, 1>); break;
+    case 2: fn = chan_branch_ring_kernel<1, 0>; break;
+    case 3: fn = chan_branch_ring_kernel<1, 1>; break;
+    case 4: fn = chan_branch_ring_kernel<2, 0>; break;
+    case 5: fn = chan_branch_ring_kernel<2, 1>; break;
+    case 6: fn = chan_branch_ring_kernel<3, 0>; break;
+    case 7: fn = chan_branch_ring_kernel<3, 1>; break;
+    case 8: fn = chan_branch_ring_kernel<4, 0>; break;
+    case 9: fn = chan_branch_ring_kernel<4, 1>; break;
     default: return cudaErrorInvalidValue;
     }
     int device = 0;
@@ -417,12 +423,8 @@ static cudaError_t ring_launch(const void* x, const float* taps, float2* u, long
     }
     int guard_frames = kR * (per_branch / kR + 1);
     const dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(gy));
-    void* args[] = {&x, &taps, &u, &n, &frames, &channels, &w, &seg_frames, &guard_frames};
-    err = cudaLaunchKernel(fn, grid, dim3(kRingThreads), args, 0, stream);
-    if (err != cudaSuccess) {
-        return err;
-    }
-    return cudaGetLastError();
+    return launch_overlapped(fn, grid, kRingThreads, 0, stream, x, taps, u, n, frames, channels, w,
+                             seg_frames, guard_frames);
 }
 
 cudaError_t chan_branch_launch(const void* x, const float* taps, void* u, long long frames,
@@ -480,9 +482,8 @@ cudaError_t chan_branch_launch(const void* x, const float* taps, void* u, long l
                 return e;
             }
         }
-        kernel<<<grid, kBranchThreads, bytes, stream>>>(x, taps, uo, n, frames, channels,
-                                                       num_taps, w, guard_frames);
-        return cudaSuccess;
+        return launch_overlapped(kernel, grid, kBranchThreads, bytes, stream, x, taps, uo, n, frames,
+                                 channels, num_taps, w, guard_frames);
     };
     switch (format * 2 + (staged ? 1 : 0)) {
     case 0: err = run(chan_branch_kernel<0, false>, 0); break;

@@ -38,6 +38,7 @@
 // behind the branch sums and those of tile k + 1 behind the drain. Every wait is a bounded
 // mbarrier wait.
 #include "chan_tc.cuh"
+#include "launch.hpp"
 #include "magnitude.cuh"
 #include "tc_common.cuh"
 #include "tmap.hpp"
@@ -247,6 +248,8 @@ chan_tc_kernel(const __grid_constant__ CUtensorMap xmap, const void* __restrict_
         tmem_alloc(smem_u32(&ctl.tmem_base), kTmemCols);
     }
     __syncthreads();
+    wait_for_stream();
+    allow_next();
     if (threadIdx.x == 0 && my_tiles > 0) {
         for (int h = 0; h < 2; ++h) {
             const uint32_t bar = smem_u32(&ctl.win_full[h]);
@@ -679,10 +682,9 @@ static cudaError_t launch_chan(const void* x, const float* taps, const void* twi
     }
     const int tiles = static_cast<int>((frames + kFrames - 1) / kFrames);
     const int grid = tiles < sms ? tiles : sms;
-    chan_tc_kernel<kTapsSmem, kMag, kFmt><<<grid, kThreads, bytes, stream>>>(
-        map, x, taps, static_cast<const uint16_t*>(twiddles),
-        z, n, frames, num_taps, tiles);
-    return cudaGetLastError();
+    return launch_overlapped(chan_tc_kernel<kTapsSmem, kMag, kFmt>, grid, kThreads, bytes, stream, map,
+                             x, taps, static_cast<const uint16_t*>(twiddles), z, n, frames,
+                             num_taps, tiles);
 }
 
 template <int kFmt>

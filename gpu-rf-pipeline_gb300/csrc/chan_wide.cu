@@ -43,6 +43,7 @@
 // group in that chain, and every branch warp waited on them.
 #include "chan_plain.cuh"
 #include "chan_wide.cuh"
+#include "launch.hpp"
 #include "magnitude.cuh"
 #include "tc_common.cuh"
 
@@ -145,6 +146,8 @@ chan_dft_kernel(const float2* __restrict__ u, const uint4* __restrict__ image,
     if (warp == kMmaWarp) {
         tmem_alloc(smem_u32(&ctl.tmem_base), kTmemCols);
     }
+    wait_for_stream();
+    allow_next();
     {
         uint4* dst = reinterpret_cast<uint4*>(smem + kOffW);
         for (uint32_t i = threadIdx.x; i < 2 * kWSplit / 16; i += kThreads) {
@@ -457,9 +460,8 @@ static cudaError_t launch_dft(const float2* u, const void* image, void* z, long 
     const long long groups = (frames + kGroup - 1) / kGroup;
     const long long cap = static_cast<long long>(sms) * occ;
     const unsigned grid = static_cast<unsigned>(groups < cap ? groups : cap);
-    kernel<<<grid, kThreads, kSmemBytes, stream>>>(u, static_cast<const uint4*>(image), z, frames,
-                                                   groups);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, grid, kThreads, kSmemBytes, stream, u,
+                             static_cast<const uint4*>(image), z, frames, groups);
 }
 
 cudaError_t chan_wide_launch(const void* x, const float* taps, const void* image, void* u,

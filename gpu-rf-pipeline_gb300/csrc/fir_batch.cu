@@ -1564,6 +1564,8 @@ cudaError_t fir_batch_plan_run(const BatchPlan* plan, cudaStream_t stream)
         return cudaSuccess;
     }
     const dim3 grid(static_cast<unsigned>(plan->grid));
+    // Launched the ordinary way: overlapped with the end of the run before it (launch.hpp), runs
+    // back to back took 1281 us each against 888 (256 captures), one alone no longer than before.
     switch (plan->stages) {
     case 6:
         fir_batch_list_kernel<6><<<grid, kThreads, plan->smem, stream>>>(plan->view);

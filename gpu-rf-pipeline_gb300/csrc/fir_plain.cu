@@ -3,6 +3,7 @@
 // for captures sharing one tap set, for captures with their own taps, and for integer input.
 #include "fir_plain.cuh"
 #include "fir_plain_tile.cuh"
+#include "launch.hpp"
 #include "ptx.cuh"
 
 #include <cuda_runtime.h>
@@ -34,6 +35,8 @@ fir_plain_kernel(const float2* __restrict__ x, const float* __restrict__ taps,
                  float2* __restrict__ y, long long n, int num_taps)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    wait_for_stream();
+    allow_next();
     plain_block_tile(x, taps, y, n, num_taps, blockIdx.x, smem);
 }
 
@@ -43,6 +46,8 @@ __global__ void __launch_bounds__(kThreads, 4)
 fir_plain_batched_kernel(PlainBatch batch, const float* __restrict__ taps, int num_taps)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    wait_for_stream();
+    allow_next();
     const int c = blockIdx.y;
     const long long n = batch.num_samples[c];
     if (static_cast<long long>(blockIdx.x) * kTile >= n) {
@@ -58,6 +63,8 @@ __global__ void __launch_bounds__(kThreads, 4)
 fir_plain_caps_kernel(const __grid_constant__ PlainCaps caps)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    wait_for_stream();
+    allow_next();
     const int block = static_cast<int>(blockIdx.x);
     int lo = 0;
     int hi = caps.count;
@@ -80,6 +87,8 @@ fir_plain_fmt_kernel(const void* __restrict__ x, const float* __restrict__ taps,
                      float2* __restrict__ y, long long n, int num_taps)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    wait_for_stream();
+    allow_next();
     plain_block_tile<kFmt>(x, taps, y, n, num_taps, blockIdx.x, smem);
 }
 
@@ -105,21 +114,37 @@ static cudaError_t ensure_smem_attr(const void* fn, size_t bytes)
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
 }
 
+// Shared memory for a launch of `blocks` tiles, and the function's opt-in to it.
+static cudaError_t spread_tiles(const void* fn, long long blocks, size_t* bytes)
+{
+    int device = 0;
+    int sms = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess ||
+        (err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) !=
+            cudaSuccess) {
+        return err;
+    }
+    *bytes = even_spread_smem(*bytes, blocks, sms, 4);
+    return ensure_smem_attr(fn, *bytes);
+}
+
 cudaError_t fir_plain_launch(const void* x, const float* taps, void* y, long long n,
                              int num_taps, cudaStream_t stream)
 {
     if (n <= 0) {
         return cudaSuccess;
     }
-    const size_t bytes = fir_plain_smem_bytes(num_taps);
-    cudaError_t err = ensure_smem_attr(reinterpret_cast<const void*>(fir_plain_kernel), bytes);
+    const long long tiles = (n + kTile - 1) / kTile;
+    size_t bytes = fir_plain_smem_bytes(num_taps);
+    const cudaError_t err =
+        spread_tiles(reinterpret_cast<const void*>(fir_plain_kernel), tiles, &bytes);
     if (err != cudaSuccess) {
         return err;
     }
-    const long long tiles = (n + kTile - 1) / kTile;
-    fir_plain_kernel<<<static_cast<unsigned>(tiles), kThreads, bytes, stream>>>(
-        static_cast<const float2*>(x), taps, static_cast<float2*>(y), n, num_taps);
-    return cudaGetLastError();
+    return launch_overlapped(fir_plain_kernel, static_cast<unsigned>(tiles), kThreads, bytes, stream,
+                             static_cast<const float2*>(x), taps, static_cast<float2*>(y), n,
+                             num_taps);
 }
 
 cudaError_t fir_plain_batched_launch(const PlainBatch& batch, int count, const float* taps,
@@ -132,15 +157,16 @@ cudaError_t fir_plain_batched_launch(const PlainBatch& batch, int count, const f
     if (longest == 0) {
         return cudaSuccess;
     }
-    const size_t bytes = fir_plain_smem_bytes(num_taps);
-    cudaError_t err =
-        ensure_smem_attr(reinterpret_cast<const void*>(fir_plain_batched_kernel), bytes);
+    const dim3 grid(static_cast<unsigned>((longest + kTile - 1) / kTile), count);
+    size_t bytes = fir_plain_smem_bytes(num_taps);
+    const cudaError_t err =
+        spread_tiles(reinterpret_cast<const void*>(fir_plain_batched_kernel),
+                     static_cast<long long>(grid.x) * count, &bytes);
     if (err != cudaSuccess) {
         return err;
     }
-    const dim3 grid(static_cast<unsigned>((longest + kTile - 1) / kTile), count);
-    fir_plain_batched_kernel<<<grid, kThreads, bytes, stream>>>(batch, taps, num_taps);
-    return cudaGetLastError();
+    return launch_overlapped(fir_plain_batched_kernel, grid, kThreads, bytes, stream, batch, taps,
+                             num_taps);
 }
 
 cudaError_t fir_plain_launch_format(int format, const void* x, const float* taps, void* y,
@@ -152,22 +178,17 @@ cudaError_t fir_plain_launch_format(int format, const void* x, const float* taps
     if (n <= 0) {
         return cudaSuccess;
     }
-    const size_t bytes = plain_layout(num_taps, format).bytes;
+    const long long tiles = (n + kTile - 1) / kTile;
+    size_t bytes = plain_layout(num_taps, format).bytes;
     const void* fn = format == 1 ? reinterpret_cast<const void*>(fir_plain_fmt_kernel<1>)
                                  : reinterpret_cast<const void*>(fir_plain_fmt_kernel<2>);
-    cudaError_t err = ensure_smem_attr(fn, bytes);
+    const cudaError_t err = spread_tiles(fn, tiles, &bytes);
     if (err != cudaSuccess) {
         return err;
     }
-    const long long tiles = (n + kTile - 1) / kTile;
-    if (format == 1) {
-        fir_plain_fmt_kernel<1><<<static_cast<unsigned>(tiles), kThreads, bytes, stream>>>(
-            x, taps, static_cast<float2*>(y), n, num_taps);
-    } else {
-        fir_plain_fmt_kernel<2><<<static_cast<unsigned>(tiles), kThreads, bytes, stream>>>(
-            x, taps, static_cast<float2*>(y), n, num_taps);
-    }
-    return cudaGetLastError();
+    return launch_overlapped(format == 1 ? fir_plain_fmt_kernel<1> : fir_plain_fmt_kernel<2>,
+                             static_cast<unsigned>(tiles), kThreads, bytes, stream, x, taps,
+                             static_cast<float2*>(y), n, num_taps);
 }
 
 cudaError_t fir_plain_caps_launch(const PlainCaps& caps, cudaStream_t stream)
@@ -180,14 +201,14 @@ cudaError_t fir_plain_caps_launch(const PlainCaps& caps, cudaStream_t stream)
     for (int c = 0; c < caps.count; ++c) {
         kmax = caps.num_taps[c] > kmax ? caps.num_taps[c] : kmax;
     }
-    const size_t bytes = fir_plain_smem_bytes(kmax);
-    cudaError_t err =
-        ensure_smem_attr(reinterpret_cast<const void*>(fir_plain_caps_kernel), bytes);
+    size_t bytes = fir_plain_smem_bytes(kmax);
+    const cudaError_t err =
+        spread_tiles(reinterpret_cast<const void*>(fir_plain_caps_kernel), tiles, &bytes);
     if (err != cudaSuccess) {
         return err;
     }
-    fir_plain_caps_kernel<<<static_cast<unsigned>(tiles), kThreads, bytes, stream>>>(caps);
-    return cudaGetLastError();
+    return launch_overlapped(fir_plain_caps_kernel, static_cast<unsigned>(tiles), kThreads, bytes,
+                             stream, caps);
 }
 
 cudaError_t fir_plain_take_fault(unsigned int* code)

@@ -46,6 +46,7 @@
 #include "fir_tc.cuh"
 #include "fir_plain.cuh"
 #include "fir_tc2.cuh"
+#include "launch.hpp"
 #include "tuning.hpp"
 #include "sample_fmt.cuh"
 #include "tc_common.cuh"
@@ -260,6 +261,8 @@ fir_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ 
         tmem_alloc(smem_u32(&ctl.tmem_base), kTmemCols);
     }
     __syncthreads();
+    wait_for_stream();
+    allow_next();
     // Scan slice q: the next tile's (q / 8 + 1) window rows (q % 8) srows .. + srows.
     auto issue_scan = [&](int q) {
         const int kn = q / kStagesPerTile + 1;
@@ -789,9 +792,8 @@ static cudaError_t launch_stages(int fmt, const void* x, const float* taps, void
     const long long blocks = (n + kB - 1) / kB;
     const int tiles = static_cast<int>((blocks + kNB - 1) / kNB);
     const int grid = tiles < sms ? tiles : sms;
-    fir_tc_kernel<S, kInt><<<grid, kThreads, bytes, stream>>>(
-        map, smap, x, taps, static_cast<float2*>(y), n, num_taps, tiles, sbufs, fmt);
-    return cudaGetLastError();
+    return launch_overlapped(fir_tc_kernel<S, kInt>, grid, kThreads, bytes, stream, map, smap, x,
+                             taps, static_cast<float2*>(y), n, num_taps, tiles, sbufs, fmt);
 }
 
 // The single-CTA form over x in format fmt (n >= one block).

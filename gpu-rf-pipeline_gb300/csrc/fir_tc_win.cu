@@ -44,6 +44,7 @@
 // every K-step); a give-up sets the fault word and every role stops.
 #include "fir_tc.cuh"
 #include "fir_tc_win.cuh"
+#include "launch.hpp"
 #include "tmap.hpp"
 
 #include <cuda.h>
@@ -74,6 +75,8 @@ fir_tcw_kernel(const __grid_constant__ CUtensorMap wmap, const void* __restrict_
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = *tmem_slot;
+    wait_for_stream();
+    allow_next();
     const tcw::TcwSingleSrc src{&wmap, tcw::WinCapture{x, y, taps, n, num_taps, 0}, num_tiles};
     tcw::tcw_pipeline<C, kFmt, 8>(src, smem, ctl, tmem, &g_fault_fir_tcw);
     if (warp == tcw::kMmaWarp) {
@@ -133,9 +136,8 @@ static cudaError_t launch_tcw(const void* x, const float* taps, void* y, long lo
     const long long blocks = (n + tcw::kB - 1) / tcw::kB;
     const int tiles = static_cast<int>((blocks + tcw::kNB - 1) / tcw::kNB);
     const int grid = tiles < sms ? tiles : sms;
-    fir_tcw_kernel<C, kFmt><<<grid, tcw::kThreads, bytes, stream>>>(
-        map, x, taps, static_cast<float2*>(y), n, num_taps, tiles);
-    return cudaGetLastError();
+    return launch_overlapped(fir_tcw_kernel<C, kFmt>, grid, tcw::kThreads, bytes, stream, map, x,
+                             taps, static_cast<float2*>(y), n, num_taps, tiles);
 }
 
 cudaError_t fir_tcw_launch(int format, const void* x, const float* taps, void* y, long long n,

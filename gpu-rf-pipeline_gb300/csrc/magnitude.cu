@@ -4,6 +4,8 @@
 // samples per step (one 16-byte load, one 8-byte store), in a grid-stride loop over a grid of a
 // few blocks per SM; an odd last sample is done on its own.
 #include "magnitude.cuh"
+#include "launch.hpp"
+#include "ptx.cuh"
 
 namespace rfx {
 namespace {
@@ -14,6 +16,8 @@ __global__ void __launch_bounds__(kThreads)
 magnitude_kernel(const float4* __restrict__ x, float2* __restrict__ mag, long long pairs,
                  long long n)
 {
+    wait_for_stream();
+    allow_next();
     const long long stride = static_cast<long long>(gridDim.x) * kThreads;
     for (long long i = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x; i < pairs;
          i += stride) {
@@ -45,9 +49,9 @@ cudaError_t magnitude_launch(const void* x, float* mag, long long n, cudaStream_
     const long long want = (pairs + kThreads - 1) / kThreads;
     const long long cap = static_cast<long long>(sms) * 8;
     const int grid = static_cast<int>(want < 1 ? 1 : (want < cap ? want : cap));
-    magnitude_kernel<<<grid, kThreads, 0, stream>>>(static_cast<const float4*>(x),
-                                                     reinterpret_cast<float2*>(mag), pairs, n);
-    return cudaGetLastError();
+    return launch_overlapped(magnitude_kernel, grid, kThreads, 0, stream,
+                             static_cast<const float4*>(x), reinterpret_cast<float2*>(mag), pairs,
+                             n);
 }
 
 }  // namespace rfx

@@ -179,6 +179,22 @@ __device__ __forceinline__ void cluster_sync_all()
                  "barrier.cluster.wait.acquire;" ::: "memory");
 }
 
+// ---- overlap with the neighbouring kernels of the stream (launch.hpp) ------------------
+
+// Waits until every earlier kernel of the stream has completed and its writes are visible (the
+// hardware completes it; at once for a kernel launched in the ordinary way).
+__device__ __forceinline__ void wait_for_stream()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Lets the next kernel of the stream be scheduled once every block of this one has come here.
+// After wait_for_stream(), so that no more than two kernels of a stream are ever in flight.
+__device__ __forceinline__ void allow_next()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- bulk copies (TMA engine, no tensor map) -------------------------------------------
 
 // global -> shared, completion counted on `bar` in bytes. dst/src 16-byte aligned, bytes % 16 == 0.
