@@ -11,11 +11,19 @@ namespace rfx {
 struct TcConfig {
     int tile_blocks;  // 128-output blocks per tile: 96 = one CTA per tile (fir_tc.cu),
                       // 192 = a CTA pair per tile of 96 256-output blocks (fir_tc2.cu),
-                      // 48 = the resident-window form, 2 to 1025 taps (fir_tc_win.cu)
+                      // 8, 16, 24, 32 or 48 = the resident-window form, 2 to 385 taps
+                      // (fir_tc_win.cu)
     int stages;       // operand ring depth cap (the largest that fits is used)
 };
 constexpr int kTcPairTile = 192;
-constexpr int kTcWindowTile = 48;
+constexpr int kTcWindowTile = 48;   // the largest of the resident-window form
+
+// Whether a tile shape is the resident-window form's.
+constexpr bool is_window_tile(int tile_blocks)
+{
+    return tile_blocks == 8 || tile_blocks == 16 || tile_blocks == 24 || tile_blocks == 32 ||
+           tile_blocks == 48;
+}
 
 constexpr int kTcBatchMax = 4096;
 
@@ -27,13 +35,14 @@ cudaError_t fir_tc_launch(const void* x, const float* taps, void* y, long long n
                           TcConfig config, cudaStream_t stream);
 cudaError_t fir_tc_take_fault(unsigned int* code);
 
-// The resident-window form (fir_tc_win.cu): 2 to 1025 taps, tiles of 48 blocks whose whole input
-// window arrives by one TMA copy; format 0 cf32, 1 ci16, 2 ci8 (decoded in the load stage, the
+// The resident-window form (fir_tc_win.cu): 2 to 385 taps, tiles of `tile_blocks` blocks whose
+// whole input window arrives by one TMA copy; format 0 cf32, 1 ci16, 2 ci8 (decoded in the load stage, the
 // same bits as over the converted samples). n >= 128.
 bool fir_tcw_supported(int num_taps);
-long long fir_tcw_tile_outputs();
-cudaError_t fir_tcw_launch(int format, const void* x, const float* taps, void* y, long long n,
-                           int num_taps, cudaStream_t stream);
+cudaError_t fir_tcw_launch(int tile_blocks, int format, const void* x, const float* taps, void* y,
+                           long long n, int num_taps, cudaStream_t stream);
+// The tile the form takes for a capture of n samples by the built-in rule.
+int fir_tcw_tile_blocks(int num_taps, long long n);
 cudaError_t fir_tcw_take_fault(unsigned int* code);
 
 // The same FIR over integer I/Q input decoded in the load stage (format 1 = ci16, 2 = ci8; 0 =

@@ -5,8 +5,9 @@
 //
 // Blocks of B = 128 outputs; a block reaches back C = floor((K + 126) / 128) blocks (1 to 3):
 //   Y[:, j] = sum_{c=0}^{C} T_c X[:, j - c],   T_c(r, s) = h[cB + r - s]  (0 outside [0, K)).
-// A tile is NB = 48 blocks (6144 outputs); its input window is blocks j0 - C .. j0 + 47. The
-// GEMM per tile is D (128 x 96) += A (128 x 16) B (16 x 96) over K-steps (c, st): A is a
+// A tile is NB blocks, 48 (6144 outputs) in long captures and 8 to 32 where smaller tiles spread
+// a short one over more SMs (fir_tcw_tile_blocks); its input window is blocks j0 - C .. j0 + NB - 1.
+// The GEMM per tile is D (128 x 2 NB) += A (128 x 16) B (16 x 2 NB) over K-steps (c, st): A is a
 // descriptor into the tap strip (fir_tc.cu's layout: output rows stored reversed, so every 8 x 8
 // core matrix of every T_c is one strip element), B the FP16 planes of K-step st (16 samples of
 // each window row, N index 2 j + {0: I, 1: Q}). Chunk C of a K-step whose taps are all zero
@@ -37,7 +38,7 @@
 //
 // Roles (640 threads): warp 0 copies windows; warp 1 owns tensor memory and issues the MMAs (the
 // warp runs the loop, one elected lane issues); warps 2-9 produce (FP16 hi/lo planes); warps
-// 10-17 drain (warp w reads TMEM lane quarter w % 4, the columns of blocks 24 h .. 24 h + 23
+// 10-17 drain (warp w reads TMEM lane quarter w % 4, the columns of half h of the tile's blocks
 // with h = (w - 10) / 4); warps 18-19 scan windows. Every wait is an mbarrier wait bounded in
 // time, polled by every lane of a waiting warp (measured: lane 0 polling alone and handing the
 // result to the warp by a shuffle took 18 us longer at 63 taps, the hand-off latency landing on
@@ -57,7 +58,7 @@ static __device__ unsigned int g_fault_fir_tcw;
 // wmap: x as rows of 256 components (one 128-sample block per row, full blocks only), boxes
 // of 256 components x (48 + C) rows (one tile window). kFmt: 0 cf32, 1 ci16, 2 ci8 (the copy
 // moves the components as stored; the producers decode them).
-template <int C, int kFmt>
+template <int C, int kFmt, int NB>
 __global__ void __launch_bounds__(tcw::kThreads, 1)
 fir_tcw_kernel(const __grid_constant__ CUtensorMap wmap, const void* __restrict__ x,
                const float* __restrict__ taps, float2* __restrict__ y, long long n, int num_taps,
@@ -78,7 +79,7 @@ fir_tcw_kernel(const __grid_constant__ CUtensorMap wmap, const void* __restrict_
     wait_for_stream();
     allow_next();
     const tcw::TcwSingleSrc src{&wmap, tcw::WinCapture{x, y, taps, n, num_taps, 0}, num_tiles};
-    tcw::tcw_pipeline<C, kFmt, 8>(src, smem, ctl, tmem, &g_fault_fir_tcw);
+    tcw::tcw_pipeline<C, kFmt, 8, tcw::TcwSingleSrc, 2, NB>(src, smem, ctl, tmem, &g_fault_fir_tcw);
     if (warp == tcw::kMmaWarp) {
         tc::tmem_dealloc(tmem, tcw::kTmemCols);
     }
@@ -90,14 +91,45 @@ bool fir_tcw_supported(int num_taps)
            tcw::win_layout((num_taps + tcw::kB - 2) / tcw::kB, 8, 1, 4).bytes <= tcw::kSmemMax;
 }
 
-long long fir_tcw_tile_outputs() { return static_cast<long long>(tcw::kNB) * tcw::kB; }
+// Tile by the time it takes the busiest SM: a first tile through the whole pipeline, whose latency
+// grows with the tile, then the others at the pipeline's rate, a step plus the blocks. Fitted to
+// times (us, 63 / 255 / 385 taps): one tile of 8, 16, 24, 32, 48 blocks 4.9 / 6.3 / 7.1, 5.1 / 6.5
+// / 7.4, 5.8 / 7.0 / 7.9, 6.0 / 7.4 / 8.3, 6.8 / 8.5 / 9.4; each further tile 1.6 / 2.4 / 3.1 (8
+// blocks) to 2.6 / 3.5 / 4.4 (48). So short captures take small tiles on more SMs (2^16 samples, 63
+// taps: 6.8 -> 4.9), middling ones the tile that fills the last round (2^20 samples, 255 taps: 11.9
+// -> 10.8), long ones the largest.
+int fir_tcw_tile_blocks(int num_taps, long long n)
+{
+    int device = 0;
+    int sms = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        sms < 1) {
+        cudaGetLastError();
+        sms = 152;
+    }
+    const int C = (num_taps + tcw::kB - 2) / tcw::kB;
+    const long long blocks = (n + tcw::kB - 1) / tcw::kB;
+    int best = kTcWindowTile;
+    double best_us = 1e30;
+    for (int nb : {48, 32, 24, 16, 8}) {
+        const long long tiles = (blocks + nb - 1) / nb;
+        const double rounds = static_cast<double>((tiles + sms - 1) / sms);
+        const double us = 0.047 * nb + (rounds - 1.0) * (0.65 + 0.72 * C + 0.03 * nb);
+        if (us < best_us) {
+            best_us = us;
+            best = nb;
+        }
+    }
+    return best;
+}
 
-template <int C, int kFmt>
+template <int C, int kFmt, int NB>
 static cudaError_t launch_tcw(const void* x, const float* taps, void* y, long long n, int num_taps,
                               cudaStream_t stream)
 {
     constexpr int es = tc::component_bytes(kFmt);
-    const tcw::Layout lay = tcw::win_layout(C, 8, 1, es);
+    const tcw::Layout lay = tcw::win_layout(C, 8, 1, es, NB);
     if (lay.bytes > tcw::kSmemMax) {
         return cudaErrorInvalidValue;
     }
@@ -119,7 +151,7 @@ static cudaError_t launch_tcw(const void* x, const float* taps, void* y, long lo
     if (bytes > static_cast<uint32_t>(optin)) {
         return cudaErrorInvalidValue;
     }
-    err = cudaFuncSetAttribute(fir_tcw_kernel<C, kFmt>,
+    err = cudaFuncSetAttribute(fir_tcw_kernel<C, kFmt, NB>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(bytes));
     if (err != cudaSuccess) {
@@ -129,34 +161,55 @@ static cudaError_t launch_tcw(const void* x, const float* taps, void* y, long lo
     // is a tile window.
     CUtensorMap map;
     err = encode_rows(&map, x, es, n / tcw::kB, 2 * tcw::kB, 2 * tcw::kB,
-                      static_cast<uint32_t>(tcw::kNB + C));
+                      static_cast<uint32_t>(NB + C));
     if (err != cudaSuccess) {
         return err;
     }
     const long long blocks = (n + tcw::kB - 1) / tcw::kB;
-    const int tiles = static_cast<int>((blocks + tcw::kNB - 1) / tcw::kNB);
+    const int tiles = static_cast<int>((blocks + NB - 1) / NB);
     const int grid = tiles < sms ? tiles : sms;
-    return launch_overlapped(fir_tcw_kernel<C, kFmt>, grid, tcw::kThreads, bytes, stream, map, x,
+    return launch_overlapped(fir_tcw_kernel<C, kFmt, NB>, grid, tcw::kThreads, bytes, stream, map, x,
                              taps, static_cast<float2*>(y), n, num_taps, tiles);
 }
 
-cudaError_t fir_tcw_launch(int format, const void* x, const float* taps, void* y, long long n,
-                           int num_taps, cudaStream_t stream)
+template <int C, int NB>
+static cudaError_t launch_formats(int format, const void* x, const float* taps, void* y,
+                                  long long n, int num_taps, cudaStream_t stream)
+{
+    switch (format) {
+    case 0: return launch_tcw<C, 0, NB>(x, taps, y, n, num_taps, stream);
+    case 1: return launch_tcw<C, 1, NB>(x, taps, y, n, num_taps, stream);
+    case 2: return launch_tcw<C, 2, NB>(x, taps, y, n, num_taps, stream);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int NB>
+static cudaError_t launch_reach(int format, const void* x, const float* taps, void* y, long long n,
+                                int num_taps, cudaStream_t stream)
+{
+    switch ((num_taps + tcw::kB - 2) / tcw::kB) {
+    case 1: return launch_formats<1, NB>(format, x, taps, y, n, num_taps, stream);
+    case 2: return launch_formats<2, NB>(format, x, taps, y, n, num_taps, stream);
+    case 3: return launch_formats<3, NB>(format, x, taps, y, n, num_taps, stream);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t fir_tcw_launch(int tile_blocks, int format, const void* x, const float* taps, void* y,
+                           long long n, int num_taps, cudaStream_t stream)
 {
     if (n < tcw::kB || !fir_tcw_supported(num_taps)) {
         return cudaErrorInvalidValue;
     }
-    const int C = (num_taps + tcw::kB - 2) / tcw::kB;
-    if (format < 0 || format > 2) {
-        return cudaErrorInvalidValue;
+    switch (tile_blocks) {
+    case 8: return launch_reach<8>(format, x, taps, y, n, num_taps, stream);
+    case 16: return launch_reach<16>(format, x, taps, y, n, num_taps, stream);
+    case 24: return launch_reach<24>(format, x, taps, y, n, num_taps, stream);
+    case 32: return launch_reach<32>(format, x, taps, y, n, num_taps, stream);
+    case 48: return launch_reach<48>(format, x, taps, y, n, num_taps, stream);
+    default: return cudaErrorInvalidValue;
     }
-    static cudaError_t (*const launchers[tcw::kCMax][3])(const void*, const float*, void*,
-                                                          long long, int, cudaStream_t) = {
-        {launch_tcw<1, 0>, launch_tcw<1, 1>, launch_tcw<1, 2>},
-        {launch_tcw<2, 0>, launch_tcw<2, 1>, launch_tcw<2, 2>},
-        {launch_tcw<3, 0>, launch_tcw<3, 1>, launch_tcw<3, 2>},
-    };
-    return launchers[C - 1][format](x, taps, y, n, num_taps, stream);
 }
 
 cudaError_t fir_tcw_take_fault(unsigned int* code)

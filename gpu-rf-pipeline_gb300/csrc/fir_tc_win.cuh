@@ -24,10 +24,9 @@ namespace tcw {
 using namespace tc;
 
 constexpr int kB = 128;                   // outputs per block = MMA M
-constexpr int kNB = 48;                   // blocks per tile; MMA N = 2 * kNB
-constexpr int kN = 2 * kNB;
+constexpr int kNB = 48;                   // blocks per tile, at most; MMA N = 2 * blocks
+constexpr int kN = 2 * kNB;               // columns of an accumulator
 constexpr int kCMax = 3;                  // blocks a block reaches back to, at most (385 taps)
-constexpr int kRowsMax = kNB + kCMax;     // window rows per tile, at most
 constexpr int kSteps = kB / 16;           // K-steps of 16 samples per tile
 constexpr int kWins = 3;                  // window buffers
 constexpr int kHGroup = 18;               // MMAs per H accumulation, at most
@@ -44,9 +43,7 @@ constexpr int kScanWarps = 2;
 constexpr int kThreads = (kFirstScanWarp + kScanWarps) * 32;
 constexpr uint32_t kTmemCols = 512;       // H0, H1, X0, X1 of kN columns each: 384 used
 constexpr uint32_t kXCol = 2 * kN;        // first column of X0
-constexpr uint32_t kIdesc = idesc_f16(kB, kN);
 constexpr uint32_t kSmemMax = 227u * 1024u;
-static_assert(kNB % 16 == 0, "a drain warp reads its kNB columns 16 at a time");
 
 // One capture as the pipeline sees it.
 struct WinCapture {
@@ -70,10 +67,10 @@ struct Layout {
     uint32_t stages0, win0, bytes;
 };
 
-__host__ __device__ inline Layout win_layout(int C, int stages, int strips, int es)
+__host__ __device__ inline Layout win_layout(int C, int stages, int strips, int es, int nb = kNB)
 {
     Layout l;
-    const int rows = kNB + C;
+    const int rows = nb + C;
     l.tcount = 16 * C + 31;
     l.pitch = static_cast<uint32_t>(2 * rows) * 16u + 16u;
     l.split = 2u * l.pitch;
@@ -232,14 +229,17 @@ __device__ __forceinline__ void build_strip(uint32_t hi, uint32_t lo, const floa
 // warps beyond the roles return at the final barrier) and returns after a block barrier.
 // With a list of captures (kMulti) the caller invalidates the control block's barriers before
 // the memory is used for anything else (tcw_release).
-template <int C, int kFmt, int S, class Src, int kStrips = 2>
+// NB: blocks per tile (a multiple of eight).
+template <int C, int kFmt, int S, class Src, int kStrips = 2, int NB = kNB>
 __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem, Ctrl& ctl,
                                              uint32_t tmem, unsigned int* fault)
 {
     constexpr bool kMulti = Src::kMulti;
     constexpr int es = component_bytes(kFmt);
     constexpr uint32_t kPairBytes = 4u * es;   // two samples as stored
-    constexpr int rows = kNB + C;
+    constexpr int rows = NB + C;
+    constexpr uint32_t kIdesc = idesc_f16(kB, 2 * NB);
+    static_assert(NB % 8 == 0 && NB <= kNB, "MMA N = 2 NB is a multiple of 16, at most kN");
     constexpr int hks = kSteps < kHGroup / (C + 1) ? kSteps : kHGroup / (C + 1);
     constexpr int groups = (kSteps + hks - 1) / hks;
     constexpr int wins = kWins;
@@ -253,7 +253,7 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
     static_assert(hks >= 1, "an H group holds at least one K-step");
     static_assert(S == 4 || S == 8, "4 or 8 operand stages");
     static_assert(kSteps % kGroup == 0, "producer groups");
-    const Layout lay = win_layout(C, stages, kMulti ? kStrips : 1, es);
+    const Layout lay = win_layout(C, stages, kMulti ? kStrips : 1, es, NB);
     // The warp index through a shuffle: provably the same on every lane of a warp, so values
     // derived from it in a role's loop can stay in uniform registers.
     const int warp = __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0);
@@ -270,7 +270,7 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
         const uint32_t bar = smem_u32(&ctl.win_full[k % wins]);
         mbar_arrive_expect_tx(bar, lay.win);
         tma_load_2d(sbase + lay.win0 + static_cast<uint32_t>(k % wins) * lay.win,
-                    src.tmap(copy_cursor.idx), 0, static_cast<int>(t * kNB - C), bar);
+                    src.tmap(copy_cursor.idx), 0, static_cast<int>(t * NB - C), bar);
     };
     auto strip_hi = [&](int slot) {
         return sbase + lay.taps0 + static_cast<uint32_t>(slot) * lay.strip;
@@ -556,20 +556,30 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
     } else if (warp < kFirstScanWarp) {
         // ---- drain warps: H groups into running sums, then X, scaled, stored ----------------
         const int quarter = warp & 3;
-        const int half = (warp - kFirstDrainWarp) >> 2;        // blocks kNB/2 half .. + kNB/2 - 1
+        const int half = (warp - kFirstDrainWarp) >> 2;        // blocks NB/2 half .. + NB/2 - 1
         const int r = kB - 1 - (quarter * 32 + lane);          // output row of this TMEM lane
         const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) +
-                                   static_cast<uint32_t>(half * kNB);
-        float acc[groups > 1 ? kNB : 1];
+                                   static_cast<uint32_t>(half * NB);
+        float acc[groups > 1 ? NB : 1];
 #pragma unroll
-        for (int i = 0; i < (groups > 1 ? kNB : 1); ++i) {
+        for (int i = 0; i < (groups > 1 ? NB : 1); ++i) {
             acc[i] = 0.0f;
         }
-        // Adds this lane's kNB columns of the accumulator at column `col` into acc.
+        // Adds this lane's NB columns of the accumulator at column `col` into acc, 16 at a time
+        // and the last 8 where 16 do not divide them.
         auto add_columns = [&](uint32_t col) {
             if constexpr (groups > 1) {
+                if constexpr (NB % 16 != 0) {
+                    uint32_t tt[8];
+                    tmem_ld8(lane_addr + col + static_cast<uint32_t>(NB - 8), tt);
+                    tmem_wait_ld();
 #pragma unroll
-                for (int c16 = 0; c16 < kNB / 16; ++c16) {
+                    for (int i = 0; i < 8; ++i) {
+                        acc[NB - 8 + i] += __uint_as_float(tt[i]);
+                    }
+                }
+#pragma unroll
+                for (int c16 = 0; c16 < NB / 16; ++c16) {
                     uint32_t tt[16];
                     tmem_ld16(lane_addr + col + static_cast<uint32_t>(c16 * 16), tt);
                     tmem_wait_ld();
@@ -589,7 +599,7 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
             // The capture's output and length in registers for the tile's stores.
             float2* const cap_y = src.capture(cur.idx).y;
             const long long cap_n = src.capture(cur.idx).n;
-            const long long jb0 = t * kNB + half * (kNB / 2);
+            const long long jb0 = t * NB + half * (NB / 2);
             if constexpr (groups == 1) {
                 // One H group per tile: H and X read side by side, summed and stored per 16
                 // columns (no running sums held across the tile).
@@ -607,16 +617,11 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
                 const float fb = exp2i(shift - shift / 2);
                 const uint32_t hcol = static_cast<uint32_t>(g & 1) * kN;
                 const uint32_t xcol = kXCol + static_cast<uint32_t>(k & 1) * kN;
+                // Outputs of `blocks` blocks from block jb0 + b0 on, summed from th and tx.
+                auto store = [&](const uint32_t* th, const uint32_t* tx, int b0, int blocks) {
 #pragma unroll
-                for (int c16 = 0; c16 < kNB / 16; ++c16) {
-                    uint32_t th[16];
-                    uint32_t tx[16];
-                    tmem_ld16(lane_addr + hcol + static_cast<uint32_t>(c16 * 16), th);
-                    tmem_ld16(lane_addr + xcol + static_cast<uint32_t>(c16 * 16), tx);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const long long o = (jb0 + c16 * 8 + i) * kB + r;
+                    for (int i = 0; i < blocks; ++i) {
+                        const long long o = (jb0 + b0 + i) * kB + r;
                         if (o < cap_n) {
                             const float re =
                                 __uint_as_float(th[2 * i]) + __uint_as_float(tx[2 * i]);
@@ -625,6 +630,23 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
                             cap_y[o] = make_float2(re * fa * fb, im * fa * fb);
                         }
                     }
+                };
+#pragma unroll
+                for (int c16 = 0; c16 < NB / 16; ++c16) {
+                    uint32_t th[16];
+                    uint32_t tx[16];
+                    tmem_ld16(lane_addr + hcol + static_cast<uint32_t>(c16 * 16), th);
+                    tmem_ld16(lane_addr + xcol + static_cast<uint32_t>(c16 * 16), tx);
+                    tmem_wait_ld();
+                    store(th, tx, c16 * 8, 8);
+                }
+                if constexpr (NB % 16 != 0) {
+                    uint32_t th[8];
+                    uint32_t tx[8];
+                    tmem_ld8(lane_addr + hcol + static_cast<uint32_t>(NB - 8), th);
+                    tmem_ld8(lane_addr + xcol + static_cast<uint32_t>(NB - 8), tx);
+                    tmem_wait_ld();
+                    store(th, tx, NB / 2 - 4, 4);
                 }
                 fence_before();
                 __syncwarp();
@@ -673,7 +695,7 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
             const float fb = exp2i(shift - shift / 2);
             if constexpr (groups > 1) {
 #pragma unroll
-                for (int i = 0; i < kNB / 2; ++i) {
+                for (int i = 0; i < NB / 2; ++i) {
                     const long long o = (jb0 + i) * kB + r;
                     if (o < cap_n) {
                         cap_y[o] = make_float2(acc[2 * i] * fa * fb, acc[2 * i + 1] * fa * fb);
@@ -726,7 +748,7 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
             // captures this happens once per capture: the barrier's phase counts them.
             const long long full_blocks = cap.n / kB;
             const int tail = static_cast<int>(cap.n - full_blocks * kB);
-            const long long rel = full_blocks - (t * kNB - C);
+            const long long rel = full_blocks - (t * NB - C);
             if (tail > 0 && rel >= 0 && rel < rows) {   // uniform across the scan warps
                 const uint32_t row = win + static_cast<uint32_t>(rel) * 256u * es;
                 for (int i = stid; i < tail; i += kScanWarps * 32) {

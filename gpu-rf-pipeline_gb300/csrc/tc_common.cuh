@@ -22,7 +22,7 @@ __device__ __forceinline__ unsigned long long smem_desc(uint32_t addr, uint32_t 
 }
 
 // Instruction descriptor of kind::f16 with FP16 A and B (both K-major) and FP32 D.
-constexpr uint32_t idesc_f16(int m, int n)
+__host__ __device__ constexpr uint32_t idesc_f16(int m, int n)
 {
     return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }

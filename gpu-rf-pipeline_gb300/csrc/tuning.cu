@@ -298,7 +298,8 @@ TcConfig tuned_fir_tc_config(int num_taps, long long n)
         return e.config;
     }
     // The resident-window form where it applies (one copy of each window, no scan slices).
-    return fir_tcw_supported(num_taps) ? TcConfig{kTcWindowTile, 4} : TcConfig{96, 6};
+    return fir_tcw_supported(num_taps) ? TcConfig{fir_tcw_tile_blocks(num_taps, n), 4}
+                                       : TcConfig{96, 6};
 }
 
 // Built-in rule: at 64 channels the fused FP32 kernel (chan_fused.cuh) where the tensor-core form
@@ -344,7 +345,9 @@ extern "C" int rfx_autotune_fir(int impl, int num_taps, int64_t num_samples, dou
             candidates.push_back({RFX_FIR_TC, TcConfig{kTcPairTile, st}});
         }
         if (fir_tcw_supported(num_taps)) {
-            candidates.push_back({RFX_FIR_TC, TcConfig{kTcWindowTile, 4}});
+            for (int nb : {8, 16, 24, 32, 48}) {
+                candidates.push_back({RFX_FIR_TC, TcConfig{nb, 4}});
+            }
         }
     }
     FirEntry best{RFX_FIR_PLAIN, TcConfig{96, 6}, 1e30};
