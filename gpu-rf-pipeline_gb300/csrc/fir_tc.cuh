@@ -41,6 +41,11 @@ cudaError_t fir_tc_take_fault(unsigned int* code);
 bool fir_tcw_supported(int num_taps);
 cudaError_t fir_tcw_launch(int tile_blocks, int format, const void* x, const float* taps, void* y,
                            long long n, int num_taps, cudaStream_t stream);
+// Up to kTcSharedMax captures sharing one tap set (cf32, each of at least 128 samples, none
+// touching what another writes) in one launch.
+constexpr int kTcSharedMax = 64;
+cudaError_t fir_tcw_shared_launch(const void* const* x, void* const* y, const int64_t* n, int count,
+                                  const float* taps, int num_taps, cudaStream_t stream);
 // The tile the form takes for a capture of n samples by the built-in rule.
 int fir_tcw_tile_blocks(int num_taps, long long n);
 cudaError_t fir_tcw_take_fault(unsigned int* code);

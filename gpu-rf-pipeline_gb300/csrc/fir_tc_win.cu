@@ -51,6 +51,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+
 namespace rfx {
 
 static __device__ unsigned int g_fault_fir_tcw;
@@ -80,6 +81,31 @@ fir_tcw_kernel(const __grid_constant__ CUtensorMap wmap, const void* __restrict_
     allow_next();
     const tcw::TcwSingleSrc src{&wmap, tcw::WinCapture{x, y, taps, n, num_taps, 0}, num_tiles};
     tcw::tcw_pipeline<C, kFmt, 8, tcw::TcwSingleSrc, 2, NB>(src, smem, ctl, tmem, &g_fault_fir_tcw);
+    if (warp == tcw::kMmaWarp) {
+        tc::tmem_dealloc(tmem, tcw::kTmemCols);
+    }
+}
+
+// Several cf32 captures with one tap set (each tile as in fir_tcw_kernel, so the same bits).
+template <int C, int NB>
+__global__ void __launch_bounds__(tcw::kThreads, 1)
+fir_tcw_shared_kernel(const __grid_constant__ tcw::SharedCaptures list)
+{
+    extern __shared__ __align__(1024) unsigned char smem[];
+    tcw::Ctrl& ctl = *reinterpret_cast<tcw::Ctrl*>(smem);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 1020);
+    const int warp = threadIdx.x >> 5;
+    if (warp == tcw::kMmaWarp) {
+        tc::tmem_alloc(smem_u32(tmem_slot), tcw::kTmemCols);
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = *tmem_slot;
+    wait_for_stream();
+    allow_next();
+    const tcw::TcwSharedSrc src{list};
+    tcw::tcw_pipeline<C, 0, 8, tcw::TcwSharedSrc, 1, NB>(src, smem, ctl, tmem, &g_fault_fir_tcw);
     if (warp == tcw::kMmaWarp) {
         tc::tmem_dealloc(tmem, tcw::kTmemCols);
     }
@@ -209,6 +235,81 @@ cudaError_t fir_tcw_launch(int tile_blocks, int format, const void* x, const flo
     case 32: return launch_reach<32>(format, x, taps, y, n, num_taps, stream);
     case 48: return launch_reach<48>(format, x, taps, y, n, num_taps, stream);
     default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int C, int NB>
+static cudaError_t launch_shared(tcw::SharedCaptures& list, int sms, cudaStream_t stream)
+{
+    const tcw::Layout lay = tcw::win_layout(C, 8, 1, 4, NB);
+    const uint32_t bytes = lay.bytes > 120u * 1024u ? lay.bytes : 120u * 1024u;
+    cudaError_t err = cudaFuncSetAttribute(fir_tcw_shared_kernel<C, NB>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           static_cast<int>(bytes));
+    if (err != cudaSuccess) {
+        return err;
+    }
+    list.tiles = 0;
+    for (int c = 0; c < list.count; ++c) {
+        tcw::WinCapture& cap = list.cap[c];
+        err = encode_rows(&list.map[c], cap.x, 4, cap.n / tcw::kB, 2 * tcw::kB, 2 * tcw::kB,
+                          static_cast<uint32_t>(NB + C));
+        if (err != cudaSuccess) {
+            return err;
+        }
+        cap.item0 = list.tiles;
+        list.tiles += static_cast<int>(((cap.n + tcw::kB - 1) / tcw::kB + NB - 1) / NB);
+    }
+    const int grid = list.tiles < sms ? list.tiles : sms;
+    return launch_overlapped(fir_tcw_shared_kernel<C, NB>, grid, tcw::kThreads, bytes, stream, list);
+}
+
+template <int NB>
+static cudaError_t launch_shared_reach(tcw::SharedCaptures& list, int num_taps, int sms,
+                                       cudaStream_t stream)
+{
+    switch ((num_taps + tcw::kB - 2) / tcw::kB) {
+    case 1: return launch_shared<1, NB>(list, sms, stream);
+    case 2: return launch_shared<2, NB>(list, sms, stream);
+    case 3: return launch_shared<3, NB>(list, sms, stream);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t fir_tcw_shared_launch(const void* const* x, void* const* y, const int64_t* n, int count,
+                                  const float* taps, int num_taps, cudaStream_t stream)
+{
+    int device = 0;
+    int sms = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess ||
+        (err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) !=
+            cudaSuccess) {
+        return err;
+    }
+    if (!fir_tcw_supported(num_taps)) {
+        return cudaErrorInvalidValue;
+    }
+    if (count < 1 || count > kTcSharedMax) {
+        return cudaErrorInvalidValue;
+    }
+    tcw::SharedCaptures list;   // 11 KB
+    list.count = count;
+    long long total = 0;
+    for (int c = 0; c < count; ++c) {
+        if (n[c] < tcw::kB) {
+            return cudaErrorInvalidValue;
+        }
+        list.cap[c] =
+            tcw::WinCapture{x[c], static_cast<float2*>(y[c]), taps, n[c], num_taps, 0};
+        total += n[c];
+    }
+    switch (fir_tcw_tile_blocks(num_taps, total)) {
+    case 8: return launch_shared_reach<8>(list, num_taps, sms, stream);
+    case 16: return launch_shared_reach<16>(list, num_taps, sms, stream);
+    case 24: return launch_shared_reach<24>(list, num_taps, sms, stream);
+    case 32: return launch_shared_reach<32>(list, num_taps, sms, stream);
+    default: return launch_shared_reach<48>(list, num_taps, sms, stream);
     }
 }
 

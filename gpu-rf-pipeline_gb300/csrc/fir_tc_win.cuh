@@ -3,6 +3,7 @@
 // (fir_batch.cu). The algorithm, its roles and their measured costs are described in
 // fir_tc_win.cu; this header holds the pipeline and the two ways it finds its tiles:
 //  * TcwSingleSrc: one capture, tile k of a block = blockIdx.x + k gridDim.x;
+//  * TcwSharedSrc: several captures with one tap set, tiles of all of them dealt out the same way;
 //  * TcwListSrc: a contiguous range of (capture, tile) work items, captures in increasing order,
 //    each with its own taps, length and tensor map (in global memory). The tap strip is then
 //    rebuilt per capture by the scan warps, into one of two strip slots or into the only one
@@ -12,6 +13,7 @@
 //    sample scale.
 #pragma once
 
+#include "fir_tc.cuh"
 #include "sample_fmt.cuh"
 #include "tc_common.cuh"
 
@@ -141,6 +143,42 @@ struct TcwSingleSrc {
     }
     __device__ const WinCapture& capture(int) const { return cap; }
     __device__ const CUtensorMap* tmap(int) const { return map; }
+    __device__ void acquire(int, int&) const {}
+};
+
+// Captures sharing one tap set, in the kernel parameters (item0: each one's first tile).
+struct SharedCaptures {
+    CUtensorMap map[kTcSharedMax];
+    WinCapture cap[kTcSharedMax];
+    int count;
+    int tiles;
+};
+
+struct TcwSharedSrc {
+    static constexpr bool kMulti = false;   // one tap strip, built once
+    const SharedCaptures& list;
+    __device__ int count() const
+    {
+        return static_cast<int>(blockIdx.x) < list.tiles
+                   ? (list.tiles - 1 - static_cast<int>(blockIdx.x)) / gridDim.x + 1
+                   : 0;
+    }
+    __device__ void locate(int k, TcwCursor& cur, long long& t) const
+    {
+        const int item = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
+        if (item >= cur.end) {
+            int i = cur.idx < 0 ? 0 : cur.idx;
+            while (i + 1 < list.count && list.cap[i + 1].item0 <= item) {
+                ++i;
+            }
+            cur.idx = i;
+            cur.item0 = list.cap[i].item0;
+            cur.end = i + 1 < list.count ? list.cap[i + 1].item0 : 0x7fffffff;
+        }
+        t = item - cur.item0;
+    }
+    __device__ const WinCapture& capture(int c) const { return list.cap[c]; }
+    __device__ const CUtensorMap* tmap(int c) const { return &list.map[c]; }
     __device__ void acquire(int, int&) const {}
 };
 

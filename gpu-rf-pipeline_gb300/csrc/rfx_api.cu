@@ -118,6 +118,13 @@ int resolve_fir_impl(int impl, int num_taps, int64_t n)
     return impl;
 }
 
+bool ranges_meet(const void* a, size_t size_a, const void* b, size_t size_b)
+{
+    const uintptr_t p = reinterpret_cast<uintptr_t>(a);
+    const uintptr_t q = reinterpret_cast<uintptr_t>(b);
+    return p < q + size_b && q < p + size_a;
+}
+
 size_t format_sample_bytes(int format) { return format == RFX_FORMAT_CF32 ? 8 : format == RFX_FORMAT_CI16 ? 4 : 2; }
 
 int check_format(int format)
@@ -386,14 +393,45 @@ int rfx_fir_batched_device(int impl, const void* const* x, void* const* y,
     }
     const int resolved = resolve_fir_impl(impl, num_taps, longest);
     if (resolved == RFX_FIR_TC) {
-        for (int c = 0; c < count; ++c) {
-            if (num_samples[c] == 0) {
-                continue;
+        // Captures of the resident-window form share launches (8 captures of 2^16 to 2^18 samples,
+        // 127 taps: 8 launches 58.8 us, one 13.0). Those too short for a tensor map or tuned to
+        // another form take one each, and so do captures that read or overwrite what another of
+        // the call writes: they run one after another.
+        const void* xs[rfx::kTcSharedMax];
+        void* ys[rfx::kTcSharedMax];
+        int64_t ns[rfx::kTcSharedMax];
+        int shared = 0;
+        for (int c = 0; c <= count; ++c) {
+            const bool window =
+                c < count && num_samples[c] >= 128 && rfx::fir_tcw_supported(num_taps) &&
+                rfx::is_window_tile(
+                    rfx::tuned_fir_tc_config(num_taps, num_samples[c]).tile_blocks);
+            bool flush = c == count || shared == rfx::kTcSharedMax;
+            for (int i = 0; i < shared && !flush; ++i) {
+                const size_t size = static_cast<size_t>(num_samples[c]) * 8u;
+                const size_t size_i = static_cast<size_t>(ns[i]) * 8u;
+                flush = ranges_meet(y[c], size, ys[i], size_i) ||
+                        ranges_meet(y[c], size, xs[i], size_i) ||
+                        ranges_meet(x[c], size, ys[i], size_i);
             }
-            const int rc = launch_fir(resolved, x[c], taps, y[c], num_samples[c], num_taps,
-                                      stream);
-            if (rc != RFX_OK) {
-                return rc;
+            if (flush && shared > 0) {
+                const cudaError_t err =
+                    rfx::fir_tcw_shared_launch(xs, ys, ns, shared, taps, num_taps, stream);
+                if (err != cudaSuccess) {
+                    return cuda_fail(err, "fir_tcw_shared_launch");
+                }
+                shared = 0;
+            }
+            if (window) {
+                xs[shared] = x[c];
+                ys[shared] = y[c];
+                ns[shared++] = num_samples[c];
+            } else if (c < count && num_samples[c] > 0) {
+                const int rc = launch_fir(resolved, x[c], taps, y[c], num_samples[c], num_taps,
+                                          stream);
+                if (rc != RFX_OK) {
+                    return rc;
+                }
             }
         }
         return RFX_OK;

@@ -55,3 +55,31 @@ def test_stream_keeps_the_whole_captures_tile(n: int) -> None:
     want = rfx.fir(dev(x), dev(h), impl="tc_split").cpu().numpy()
     got, _, _ = rfx.fir_stream(x, h, impl="tc_split", chunk=50001, depth=3)
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("k", [63, 129, 385])
+@pytest.mark.parametrize("lengths", [(128, 129, 70001), (100, 0, 5000, 127, 40000, 128 * 48),
+                                     tuple(range(200, 200 + 70 * 997, 997)), (400000, 3, 300001)])
+def test_channels_with_one_filter_match_oracle(k: int, lengths: tuple[int, ...]) -> None:
+    # More than one launch's captures, empty ones and ones below a block among them.
+    pairs = [inputs(n, k) for n in lengths]
+    h = pairs[0][1]
+    xs = [dev(x) for x, _ in pairs]
+    ys = [torch.full_like(x, 7.0) for x in xs]
+    rfx.fir_batched(xs, ys, dev(h), impl="tc_split")
+    for (x, _), y in zip(pairs, ys):
+        if x.size:
+            assert orc.normwise_error(y.cpu().numpy(), orc.fir_fast(x, h)) <= NORMWISE
+    assert rfx.device_fault() == 0
+
+
+def test_channels_that_feed_each_other_run_in_order() -> None:
+    # A channel reading another's output, and two channels writing one buffer.
+    a, h = (dev(v) for v in inputs(50000, 63))
+    b, c, d, e = (torch.zeros_like(a) for _ in range(4))
+    rfx.fir_batched([a, b, c, a, b], [b, c, d, e, e], h, impl="tc_split")
+    want = rfx.fir(rfx.fir(rfx.fir(a, h, "tc_split"), h, "tc_split"), h, "tc_split")
+    twice = rfx.fir(rfx.fir(a, h, "tc_split"), h, "tc_split")
+    err = (d - want).abs().max() / want.abs().max()
+    assert float(err) <= NORMWISE
+    assert float((e - twice).abs().max() / twice.abs().max()) <= NORMWISE

@@ -16,7 +16,7 @@ def chain(n: int, sync: bool) -> list[torch.Tensor]:
     gen = torch.Generator(device="cuda")
     gen.manual_seed(n)
     a = torch.view_as_complex(torch.randn((n, 2), generator=gen, device="cuda"))
-    b, c = torch.empty_like(a), torch.empty_like(a)
+    b, c, d = torch.empty_like(a), torch.empty_like(a), torch.empty_like(a)
     short = torch.randn(33, generator=gen, device="cuda") / 6
     long = torch.randn(700, generator=gen, device="cuda") / 26
     proto = torch.randn(512, generator=gen, device="cuda") / 23
@@ -37,11 +37,12 @@ def chain(n: int, sync: bool) -> list[torch.Tensor]:
             call(t64.launch, a, proto, c)
             call(p1024.launch, c, proto, b)
             call(rfx.magnitude_launch, b, mag)
-            call(rfx.fir_batched, [b, c], [c, a], short, "plain")
+            call(rfx.fir_batched, [b, c], [d, a], short, "plain")
+            call(rfx.fir_batched, [d, a], [c, b], short, "tc_split")
             call(rfx.fir_launch, "tc_split", c, short, a)
             a *= 1.0 / a.abs().max()
         torch.cuda.synchronize()
-        out = [a.clone(), b.clone(), c.clone(), mag.clone()]
+        out = [a.clone(), b.clone(), c.clone(), d.clone(), mag.clone()]
     return out
 
 
