@@ -835,7 +835,7 @@ cudaError_t fir_tc_launch(const void* x, const float* taps, void* y, long long n
         // Shorter than one block: the tensor map would be empty; the plain kernel is exact.
         return fir_plain_launch(x, taps, y, n, num_taps, stream);
     }
-    if (is_window_tile(config.tile_blocks) && fir_tcw_supported(num_taps)) {
+    if (fir_tcw_takes(num_taps, config.tile_blocks)) {
         return fir_tcw_launch(config.tile_blocks, 0, x, taps, y, n, num_taps, stream);
     }
     return launch_single(0, x, taps, y, n, num_taps, config.stages, stream);
@@ -859,7 +859,7 @@ cudaError_t fir_tc_launch_format(int format, const void* x, const float* taps, v
     if (n < kB) {
         return fir_plain_launch_format(format, x, taps, y, n, num_taps, stream);
     }
-    if (is_window_tile(config.tile_blocks) && fir_tcw_supported(num_taps)) {
+    if (fir_tcw_takes(num_taps, config.tile_blocks)) {
         return fir_tcw_launch(config.tile_blocks, format, x, taps, y, n, num_taps, stream);
     }
     // Otherwise integer input runs in the single-CTA form (also where cf32 runs the pair form).
@@ -875,7 +875,7 @@ long long fir_tc_tile_outputs(int num_taps, long long n, TcConfig config)
     if (config.tile_blocks == kTcPairTile && n >= 2 * kB && fir_tc2_supported(num_taps)) {
         return 96LL * 256;
     }
-    if (n >= kB && is_window_tile(config.tile_blocks) && fir_tcw_supported(num_taps)) {
+    if (n >= kB && fir_tcw_takes(num_taps, config.tile_blocks)) {
         return static_cast<long long>(config.tile_blocks) * kB;
     }
     return n < kB ? 1 : static_cast<long long>(kNB) * kB;
@@ -889,7 +889,7 @@ long long fir_tc_tile_outputs_format(int format, int num_taps, long long n, TcCo
     if (n <= 0 || n < kB || !fir_tc_supported(num_taps)) {
         return 1;
     }
-    return is_window_tile(config.tile_blocks) && fir_tcw_supported(num_taps)
+    return fir_tcw_takes(num_taps, config.tile_blocks)
                ? static_cast<long long>(config.tile_blocks) * kB
                : static_cast<long long>(kNB) * kB;
 }

@@ -11,8 +11,8 @@ namespace rfx {
 struct TcConfig {
     int tile_blocks;  // 128-output blocks per tile: 96 = one CTA per tile (fir_tc.cu),
                       // 192 = a CTA pair per tile of 96 256-output blocks (fir_tc2.cu),
-                      // 8, 16, 24, 32 or 48 = the resident-window form, 2 to 385 taps
-                      // (fir_tc_win.cu)
+                      // 8, 16, 24, 32 or 48 = the resident-window form, 2 to 385 taps, and 16,
+                      // 24 or 32 up to 1025 (fir_tc_win.cu)
     int stages;       // operand ring depth cap (the largest that fits is used)
 };
 constexpr int kTcPairTile = 192;
@@ -35,18 +35,26 @@ cudaError_t fir_tc_launch(const void* x, const float* taps, void* y, long long n
                           TcConfig config, cudaStream_t stream);
 cudaError_t fir_tc_take_fault(unsigned int* code);
 
-// The resident-window form (fir_tc_win.cu): 2 to 385 taps, tiles of `tile_blocks` blocks whose
+// The resident-window form (fir_tc_win.cu): 2 to 385 taps (fir_tcw_supported), for short captures
+// up to 1025 (fir_tcw_takes says which tiles), tiles of `tile_blocks` blocks whose
 // whole input window arrives by one TMA copy; format 0 cf32, 1 ci16, 2 ci8 (decoded in the load stage, the
 // same bits as over the converted samples). n >= 128.
 bool fir_tcw_supported(int num_taps);
+bool fir_tcw_takes(int num_taps, int tile_blocks);
 cudaError_t fir_tcw_launch(int tile_blocks, int format, const void* x, const float* taps, void* y,
                            long long n, int num_taps, cudaStream_t stream);
+// Its instances for 386 to 1025 taps (fir_tc_win_long.cu).
+constexpr int kTcWindowReach = 8;   // blocks of 128 outputs a block may reach back
+cudaError_t fir_tcw_long_launch(int tile_blocks, int format, const void* x, const float* taps,
+                                void* y, long long n, int num_taps, cudaStream_t stream);
+cudaError_t fir_tcw_long_take_fault(unsigned int* code);
 // Up to kTcSharedMax captures sharing one tap set (cf32, each of at least 128 samples, none
 // touching what another writes) in one launch.
 constexpr int kTcSharedMax = 64;
 cudaError_t fir_tcw_shared_launch(const void* const* x, void* const* y, const int64_t* n, int count,
                                   const float* taps, int num_taps, cudaStream_t stream);
-// The tile the form takes for a capture of n samples by the built-in rule.
+// The tile the form takes for a capture of n samples by the built-in rule; 0 where the form for long
+// filters (fir_tc.cu) is the faster one.
 int fir_tcw_tile_blocks(int num_taps, long long n);
 cudaError_t fir_tcw_take_fault(unsigned int* code);
 

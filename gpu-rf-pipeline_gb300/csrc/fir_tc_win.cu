@@ -43,48 +43,9 @@
 // time, polled by every lane of a waiting warp (measured: lane 0 polling alone and handing the
 // result to the warp by a shuffle took 18 us longer at 63 taps, the hand-off latency landing on
 // every K-step); a give-up sets the fault word and every role stops.
-#include "fir_tc.cuh"
-#include "fir_tc_win.cuh"
-#include "launch.hpp"
-#include "tmap.hpp"
-
-#include <cuda.h>
-#include <cuda_runtime.h>
-
+#include "fir_tc_win_kernel.cuh"
 
 namespace rfx {
-
-static __device__ unsigned int g_fault_fir_tcw;
-
-// wmap: x as rows of 256 components (one 128-sample block per row, full blocks only), boxes
-// of 256 components x (48 + C) rows (one tile window). kFmt: 0 cf32, 1 ci16, 2 ci8 (the copy
-// moves the components as stored; the producers decode them).
-template <int C, int kFmt, int NB>
-__global__ void __launch_bounds__(tcw::kThreads, 1)
-fir_tcw_kernel(const __grid_constant__ CUtensorMap wmap, const void* __restrict__ x,
-               const float* __restrict__ taps, float2* __restrict__ y, long long n, int num_taps,
-               int num_tiles)
-{
-    extern __shared__ __align__(1024) unsigned char smem[];
-    tcw::Ctrl& ctl = *reinterpret_cast<tcw::Ctrl*>(smem);
-    // The tensor-memory base travels through the last word of the control block's kilobyte.
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 1020);
-    const int warp = threadIdx.x >> 5;
-    if (warp == tcw::kMmaWarp) {
-        tc::tmem_alloc(smem_u32(tmem_slot), tcw::kTmemCols);
-    }
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tmem = *tmem_slot;
-    wait_for_stream();
-    allow_next();
-    const tcw::TcwSingleSrc src{&wmap, tcw::WinCapture{x, y, taps, n, num_taps, 0}, num_tiles};
-    tcw::tcw_pipeline<C, kFmt, 8, tcw::TcwSingleSrc, 2, NB>(src, smem, ctl, tmem, &g_fault_fir_tcw);
-    if (warp == tcw::kMmaWarp) {
-        tc::tmem_dealloc(tmem, tcw::kTmemCols);
-    }
-}
 
 // Several cf32 captures with one tap set (each tile as in fir_tcw_kernel, so the same bits).
 template <int C, int NB>
@@ -117,13 +78,16 @@ bool fir_tcw_supported(int num_taps)
            tcw::win_layout((num_taps + tcw::kB - 2) / tcw::kB, 8, 1, 4).bytes <= tcw::kSmemMax;
 }
 
-// Tile by the time it takes the busiest SM: a first tile through the whole pipeline, whose latency
-// grows with the tile, then the others at the pipeline's rate, a step plus the blocks. Fitted to
-// times (us, 63 / 255 / 385 taps): one tile of 8, 16, 24, 32, 48 blocks 4.9 / 6.3 / 7.1, 5.1 / 6.5
-// / 7.4, 5.8 / 7.0 / 7.9, 6.0 / 7.4 / 8.3, 6.8 / 8.5 / 9.4; each further tile 1.6 / 2.4 / 3.1 (8
-// blocks) to 2.6 / 3.5 / 4.4 (48). So short captures take small tiles on more SMs (2^16 samples, 63
-// taps: 6.8 -> 4.9), middling ones the tile that fills the last round (2^20 samples, 255 taps: 11.9
-// -> 10.8), long ones the largest.
+// Form and tile by the time of the busiest SM (us, a step per tile fitted to measurements on 152 SMs;
+// C = blocks reached back to). Resident window: a first tile through the whole pipeline, then one
+// step per further tile; long-filter form (96 blocks a tile): one step per tile. So short captures
+// take small tiles on more SMs, middling ones the tile that fills the last round, long ones the
+// largest tile of the window form or, beyond 385 taps, the long-filter form. Measured, 63 / 255 /
+// 385 taps: one tile of 8, 16, 24, 32, 48 blocks 4.9 / 6.3 / 7.1, 5.1 / 6.5 / 7.4, 5.8 / 7.0 / 7.9,
+// 6.0 / 7.4 / 8.3, 6.8 / 8.5 / 9.4, each further one 1.6 / 2.4 / 3.1 (8 blocks) to 2.6 / 3.5 / 4.4
+// (48); 511 / 1025 taps: 2^16 samples 7.9 / 11.0 (16 blocks) against 19.0 / 23.6 in the long-filter
+// form, 2^20 13.7 / 20.0 (32) against 20.2 / 25.0, 2^22 36.4 / 56.5 against 50.3 / 58.8, 2^23
+// 65.2 / 105.1 against 73.0 / 85.2.
 int fir_tcw_tile_blocks(int num_taps, long long n)
 {
     int device = 0;
@@ -136,78 +100,28 @@ int fir_tcw_tile_blocks(int num_taps, long long n)
     }
     const int C = (num_taps + tcw::kB - 2) / tcw::kB;
     const long long blocks = (n + tcw::kB - 1) / tcw::kB;
-    int best = kTcWindowTile;
-    double best_us = 1e30;
-    for (int nb : {48, 32, 24, 16, 8}) {
+    auto rounds = [&](int nb) {
         const long long tiles = (blocks + nb - 1) / nb;
-        const double rounds = static_cast<double>((tiles + sms - 1) / sms);
-        const double us = 0.047 * nb + (rounds - 1.0) * (0.65 + 0.72 * C + 0.03 * nb);
+        return static_cast<double>((tiles + sms - 1) / sms);
+    };
+    int best = 0;
+    double best_us = 1e30;
+    if (!fir_tcw_supported(num_taps)) {
+        const double r = rounds(96);
+        best_us = 9.0 + r * (10.3 + 0.5 * C) + (r < 3.0 ? r - 1.0 : 2.0) * 3.0;
+    }
+    for (int nb : {48, 32, 24, 16, 8}) {
+        if (!fir_tcw_takes(num_taps, nb)) {
+            continue;
+        }
+        const double us = 4.0 + 0.75 * C + (0.045 + 0.004 * C) * nb +
+                          (rounds(nb) - 1.0) * (0.75 + 0.53 * C + (0.02 + 0.007 * C) * nb);
         if (us < best_us) {
             best_us = us;
             best = nb;
         }
     }
     return best;
-}
-
-template <int C, int kFmt, int NB>
-static cudaError_t launch_tcw(const void* x, const float* taps, void* y, long long n, int num_taps,
-                              cudaStream_t stream)
-{
-    constexpr int es = tc::component_bytes(kFmt);
-    const tcw::Layout lay = tcw::win_layout(C, 8, 1, es, NB);
-    if (lay.bytes > tcw::kSmemMax) {
-        return cudaErrorInvalidValue;
-    }
-    int device = 0;
-    cudaError_t err = cudaGetDevice(&device);
-    if (err != cudaSuccess) {
-        return err;
-    }
-    int optin = 0;
-    int sms = 0;
-    if ((err = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
-                                      device)) != cudaSuccess ||
-        (err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) !=
-            cudaSuccess) {
-        return err;
-    }
-    // At least 120 KB per block keeps one block per SM: each block owns all 512 TMEM columns.
-    const uint32_t bytes = lay.bytes > 120u * 1024u ? lay.bytes : 120u * 1024u;
-    if (bytes > static_cast<uint32_t>(optin)) {
-        return cudaErrorInvalidValue;
-    }
-    err = cudaFuncSetAttribute(fir_tcw_kernel<C, kFmt, NB>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(bytes));
-    if (err != cudaSuccess) {
-        return err;
-    }
-    // x as rows of 256 components (one 128-sample block per row), full blocks only; one box
-    // is a tile window.
-    CUtensorMap map;
-    err = encode_rows(&map, x, es, n / tcw::kB, 2 * tcw::kB, 2 * tcw::kB,
-                      static_cast<uint32_t>(NB + C));
-    if (err != cudaSuccess) {
-        return err;
-    }
-    const long long blocks = (n + tcw::kB - 1) / tcw::kB;
-    const int tiles = static_cast<int>((blocks + NB - 1) / NB);
-    const int grid = tiles < sms ? tiles : sms;
-    return launch_overlapped(fir_tcw_kernel<C, kFmt, NB>, grid, tcw::kThreads, bytes, stream, map, x,
-                             taps, static_cast<float2*>(y), n, num_taps, tiles);
-}
-
-template <int C, int NB>
-static cudaError_t launch_formats(int format, const void* x, const float* taps, void* y,
-                                  long long n, int num_taps, cudaStream_t stream)
-{
-    switch (format) {
-    case 0: return launch_tcw<C, 0, NB>(x, taps, y, n, num_taps, stream);
-    case 1: return launch_tcw<C, 1, NB>(x, taps, y, n, num_taps, stream);
-    case 2: return launch_tcw<C, 2, NB>(x, taps, y, n, num_taps, stream);
-    default: return cudaErrorInvalidValue;
-    }
 }
 
 template <int NB>
@@ -222,11 +136,24 @@ static cudaError_t launch_reach(int format, const void* x, const float* taps, vo
     }
 }
 
+bool fir_tcw_takes(int num_taps, int tile_blocks)
+{
+    if (fir_tcw_supported(num_taps)) {
+        return is_window_tile(tile_blocks);
+    }
+    const int C = (num_taps + tcw::kB - 2) / tcw::kB;
+    return C > tcw::kCMax && C <= kTcWindowReach &&
+           (tile_blocks == 16 || tile_blocks == 24 || tile_blocks == 32);
+}
+
 cudaError_t fir_tcw_launch(int tile_blocks, int format, const void* x, const float* taps, void* y,
                            long long n, int num_taps, cudaStream_t stream)
 {
-    if (n < tcw::kB || !fir_tcw_supported(num_taps)) {
+    if (n < tcw::kB || !fir_tcw_takes(num_taps, tile_blocks)) {
         return cudaErrorInvalidValue;
+    }
+    if (!fir_tcw_supported(num_taps)) {
+        return fir_tcw_long_launch(tile_blocks, format, x, taps, y, n, num_taps, stream);
     }
     switch (tile_blocks) {
     case 8: return launch_reach<8>(format, x, taps, y, n, num_taps, stream);
@@ -316,11 +243,15 @@ cudaError_t fir_tcw_shared_launch(const void* const* x, void* const* y, const in
 cudaError_t fir_tcw_take_fault(unsigned int* code)
 {
     unsigned int zero = 0;
+    unsigned int more = 0;
     cudaError_t err = cudaMemcpyFromSymbol(code, g_fault_fir_tcw, sizeof(unsigned int));
-    if (err != cudaSuccess) {
+    if (err != cudaSuccess ||
+        (err = cudaMemcpyToSymbol(g_fault_fir_tcw, &zero, sizeof(unsigned int))) != cudaSuccess ||
+        (err = fir_tcw_long_take_fault(&more)) != cudaSuccess) {
         return err;
     }
-    return cudaMemcpyToSymbol(g_fault_fir_tcw, &zero, sizeof(unsigned int));
+    *code |= more;
+    return cudaSuccess;
 }
 
 }  // namespace rfx

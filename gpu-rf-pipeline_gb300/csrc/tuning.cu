@@ -298,8 +298,8 @@ TcConfig tuned_fir_tc_config(int num_taps, long long n)
         return e.config;
     }
     // The resident-window form where it applies (one copy of each window, no scan slices).
-    return fir_tcw_supported(num_taps) ? TcConfig{fir_tcw_tile_blocks(num_taps, n), 4}
-                                       : TcConfig{96, 6};
+    const int window = fir_tcw_tile_blocks(num_taps, n);
+    return window != 0 ? TcConfig{window, 4} : TcConfig{96, 6};
 }
 
 // Built-in rule: at 64 channels the fused FP32 kernel (chan_fused.cuh) where the tensor-core form
@@ -344,8 +344,8 @@ extern "C" int rfx_autotune_fir(int impl, int num_taps, int64_t num_samples, dou
         for (int st : {2, 4, 6}) {
             candidates.push_back({RFX_FIR_TC, TcConfig{kTcPairTile, st}});
         }
-        if (fir_tcw_supported(num_taps)) {
-            for (int nb : {8, 16, 24, 32, 48}) {
+        for (int nb : {8, 16, 24, 32, 48}) {
+            if (fir_tcw_takes(num_taps, nb)) {
                 candidates.push_back({RFX_FIR_TC, TcConfig{nb, 4}});
             }
         }

@@ -37,21 +37,30 @@ def test_tile_sizes_match_oracle(n: int, k: int) -> None:
     assert rfx.device_fault() == 0
 
 
+# Every reach-back of the filters beyond 385 taps, whose short captures take this form.
+@pytest.mark.parametrize("n", [128, 1025] + LENGTHS[3:])
+@pytest.mark.parametrize("k", [386, 513, 514, 641, 642, 769, 770, 897, 898, 1025])
+def test_long_filters_match_oracle(n: int, k: int) -> None:
+    test_tile_sizes_match_oracle(n, k)
+
+
 @pytest.mark.parametrize("fmt", ["ci16", "ci8"])
 @pytest.mark.parametrize("n", LENGTHS[::3])
-def test_tile_sizes_integer_input_bits(n: int, fmt: str) -> None:
+@pytest.mark.parametrize("k", [200, 600, 1025])
+def test_tile_sizes_integer_input_bits(k: int, n: int, fmt: str) -> None:
     info = np.iinfo(np.int16 if fmt == "ci16" else np.int8)
     rng = np.random.default_rng(n)
     comps = rng.integers(info.min, info.max + 1, size=2 * n).astype(info.dtype)
-    _, h = inputs(n, 200)
+    _, h = inputs(n, k)
     y = rfx.fir_format(dev(comps), dev(h), fmt, impl="tc_split")
     want = rfx.fir(dev(orc.decode(comps, fmt)), dev(h), impl="tc_split")
     assert torch.equal(torch.view_as_real(y), torch.view_as_real(want))
 
 
+@pytest.mark.parametrize("k", [300, 1025])
 @pytest.mark.parametrize("n", LENGTHS[::3])
-def test_stream_keeps_the_whole_captures_tile(n: int) -> None:
-    x, h = inputs(n, 300)
+def test_stream_keeps_the_whole_captures_tile(n: int, k: int) -> None:
+    x, h = inputs(n, k)
     want = rfx.fir(dev(x), dev(h), impl="tc_split").cpu().numpy()
     got, _, _ = rfx.fir_stream(x, h, impl="tc_split", chunk=50001, depth=3)
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
