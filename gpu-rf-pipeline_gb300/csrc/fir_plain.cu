@@ -1,12 +1,15 @@
-// Plain FP32 FIR kernels for sm_103a: one tile of 2304 outputs per block of 256 threads
-// (fir_plain_tile.cuh holds the tile function, its arithmetic and its staging), for one capture,
-// for captures sharing one tap set, for captures with their own taps, and for integer input.
+// Plain FP32 FIR kernels for sm_103a: one tile per block (fir_plain_tile.cuh holds the tile
+// function, its arithmetic and its staging), for one capture (cf32 or integer input) and for
+// captures sharing one tap set in tiles of 384 to 1792 outputs by the amount of work (tile_shape),
+// and for captures with their own taps in tiles of 2304.
 #include "fir_plain.cuh"
 #include "fir_plain_tile.cuh"
 #include "launch.hpp"
 #include "ptx.cuh"
 
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 namespace rfx {
 
@@ -15,46 +18,49 @@ static __device__ unsigned int g_fault_fir_plain;
 namespace {
 
 constexpr int kThreads = kPlainThreads;
-constexpr int kTile = kPlainTileOutputs;
 
 // One tile per block, the whole block as the tile's thread group.
-template <int kFmt = 0>
+template <int kFmt = 0, int R = kPlainOutputsPerThread, int T = kPlainThreads>
 __device__ __forceinline__ void plain_block_tile(const void* x, const float* taps, float2* y,
                                                  long long n, int num_taps, long long tile,
                                                  unsigned char* smem)
 {
     uint32_t phase = 0;
-    fir_plain_tile<kFmt>(x, taps, y, n, num_taps, tile, smem, &g_fault_fir_plain,
-                         static_cast<int>(threadIdx.x), PlainBlockSync{}, phase, true);
+    fir_plain_tile<kFmt, R, T>(x, taps, y, n, num_taps, tile, smem, &g_fault_fir_plain,
+                               static_cast<int>(threadIdx.x), PlainBlockSync{}, phase, true);
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(kThreads, 4)
-fir_plain_kernel(const float2* __restrict__ x, const float* __restrict__ taps,
+// kFmt: cf32 input, or integer I/Q (1 ci16, 2 ci8) decoded in the load stage.
+template <int kFmt, int R, int T>
+__global__ void __launch_bounds__(T, 1024 / T)
+fir_plain_kernel(const void* __restrict__ x, const float* __restrict__ taps,
                  float2* __restrict__ y, long long n, int num_taps)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     wait_for_stream();
     allow_next();
-    plain_block_tile(x, taps, y, n, num_taps, blockIdx.x, smem);
+    plain_block_tile<kFmt, R, T>(x, taps, y, n, num_taps, blockIdx.x, smem);
 }
 
 // Several captures sharing one tap set: blockIdx.y picks the capture; blocks past a shorter
 // capture's end return at once (as the project's batched kernels, src/fused.cu:141-162).
-__global__ void __launch_bounds__(kThreads, 4)
-fir_plain_batched_kernel(PlainBatch batch, const float* __restrict__ taps, int num_taps)
+template <int R, int T>
+__global__ void __launch_bounds__(T, 1024 / T)
+fir_plain_batched_kernel(const __grid_constant__ PlainBatch batch, const float* __restrict__ taps,
+                         int num_taps)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     wait_for_stream();
     allow_next();
     const int c = blockIdx.y;
     const long long n = batch.num_samples[c];
-    if (static_cast<long long>(blockIdx.x) * kTile >= n) {
+    if (static_cast<long long>(blockIdx.x) * (T * R) >= n) {
         return;
     }
-    plain_block_tile(batch.x[c], taps, static_cast<float2*>(batch.y[c]), n, num_taps, blockIdx.x,
-                     smem);
+    plain_block_tile<0, R, T>(batch.x[c], taps, static_cast<float2*>(batch.y[c]), n, num_taps,
+                              blockIdx.x, smem);
 }
 
 // Captures with their own taps: block b takes tile b - tile0[c] of the capture c whose tiles
@@ -80,20 +86,6 @@ fir_plain_caps_kernel(const __grid_constant__ PlainCaps caps)
                      caps.num_samples[lo], caps.num_taps[lo], block - caps.tile0[lo], smem);
 }
 
-// Integer I/Q input (ci16, ci8), decoded in the load stage.
-template <int kFmt>
-__global__ void __launch_bounds__(kThreads, 4)
-fir_plain_fmt_kernel(const void* __restrict__ x, const float* __restrict__ taps,
-                     float2* __restrict__ y, long long n, int num_taps)
-{
-    extern __shared__ __align__(128) unsigned char smem[];
-    wait_for_stream();
-    allow_next();
-    plain_block_tile<kFmt>(x, taps, y, n, num_taps, blockIdx.x, smem);
-}
-
-size_t fir_plain_smem_bytes(int num_taps) { return plain_layout(num_taps).bytes; }
-
 static cudaError_t ensure_smem_attr(const void* fn, size_t bytes)
 {
     // The opt-in limit only has to be raised once per function and size class; raising it to
@@ -114,81 +106,158 @@ static cudaError_t ensure_smem_attr(const void* fn, size_t bytes)
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
 }
 
-// Shared memory for a launch of `blocks` tiles, and the function's opt-in to it.
-static cudaError_t spread_tiles(const void* fn, long long blocks, size_t* bytes)
+// Shared memory for a launch of `blocks` tiles, `fit` of which fit an SM, and the function's
+// opt-in to it.
+static cudaError_t spread_tiles(const void* fn, long long blocks, int sms, int fit, size_t* bytes)
+{
+    *bytes = even_spread_smem(*bytes, blocks, sms, fit);
+    return ensure_smem_attr(fn, *bytes);
+}
+
+static cudaError_t sm_count(int* sms)
 {
     int device = 0;
+    const cudaError_t err = cudaGetDevice(&device);
+    return err == cudaSuccess
+               ? cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device)
+               : err;
+}
+
+// The tile of a launch over `outputs` outputs: threads and outputs per thread.
+struct TileShape {
+    int threads;
+    int outputs;
+};
+
+// By the time of the busiest SM, in cycles: w warps per scheduler (at least one), each R cycles of
+// a tap. Fitted to times on 152 SMs at 16 to 1025 taps: a warp alone on its scheduler takes 12.5,
+// 18.6 and 26 cycles per tap for 3, 5 and 9 outputs per thread, several share it at 12.5, 15.2,
+// 18.9 and 23.3 each (the fewer outputs, the more sample loads per tap), and no fewer than `least`
+// with staging. Measured, 1025 taps (us): 4096 samples 8.6 (3 outputs) against 25.5 for the tile of
+// 256 threads and 9 outputs that every call took, 65536 samples 11.5 (5) against 25.4, 2^18 samples
+// 20.9 (7) against 25.6; 63 taps: 10007 samples 2.4 against 4.0, 2^24 75.6 (9 outputs, 128 threads)
+// against 78.1.
+static TileShape tile_shape(long long outputs, int num_taps, int sms)
+{
+    struct Candidate {
+        TileShape shape;
+        double per_tap;      // cycles per tap and warp of a scheduler
+        double alone;        // cycles per tap of one warp
+        double least;        // cycles per warp
+        double floor_cycles; // of the launch
+    };
+    static constexpr Candidate kCandidates[] = {
+        {{128, 9}, 23.3, 26.0, 780.0, 2500.0},
+        {{256, 7}, 18.9, 18.9, 620.0, 3100.0},
+        {{128, 5}, 15.2, 18.6, 480.0, 1400.0},
+        {{128, 3}, 12.5, 12.5, 460.0, 1500.0},
+    };
+    TileShape best = kCandidates[0].shape;
+    double best_cycles = 1e300;
+    for (const Candidate& c : kCandidates) {
+        const long long tile = static_cast<long long>(c.shape.threads) * c.shape.outputs;
+        const long long per_sm = ((outputs + tile - 1) / tile + sms - 1) / sms;
+        const double w = static_cast<double>(per_sm) * c.shape.threads / 128.0;
+        const double tap = w > 1.0 ? w * c.per_tap : c.alone;
+        double cycles = num_taps * tap;
+        cycles = cycles > w * c.least ? cycles : w * c.least;
+        cycles = cycles > c.floor_cycles ? cycles : c.floor_cycles;
+        if (cycles < best_cycles) {
+            best_cycles = cycles;
+            best = c.shape;
+        }
+    }
+    return best;
+}
+
+// Calls run(R, T) as integral constants for a shape.
+template <class Run>
+static cudaError_t with_shape(TileShape shape, Run run)
+{
+    using std::integral_constant;
+    switch (shape.outputs) {
+    case 3: return run(integral_constant<int, 3>{}, integral_constant<int, 128>{});
+    case 5: return run(integral_constant<int, 5>{}, integral_constant<int, 128>{});
+    case 7: return run(integral_constant<int, 7>{}, integral_constant<int, 256>{});
+    default: return run(integral_constant<int, 9>{}, integral_constant<int, 128>{});
+    }
+}
+
+template <int kFmt>
+static cudaError_t launch_plain(const void* x, const float* taps, void* y, long long n,
+                                int num_taps, cudaStream_t stream)
+{
+    if (n <= 0) {
+        return cudaSuccess;
+    }
     int sms = 0;
-    cudaError_t err = cudaGetDevice(&device);
-    if (err != cudaSuccess ||
-        (err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) !=
-            cudaSuccess) {
+    const cudaError_t err = sm_count(&sms);
+    if (err != cudaSuccess) {
         return err;
     }
-    *bytes = even_spread_smem(*bytes, blocks, sms, 4);
-    return ensure_smem_attr(fn, *bytes);
+    return with_shape(tile_shape(n, num_taps, sms), [&](auto r, auto t) {
+        constexpr int R = decltype(r)::value;
+        constexpr int T = decltype(t)::value;
+        auto kernel = fir_plain_kernel<kFmt, R, T>;
+        const long long tiles = (n + T * R - 1) / (T * R);
+        size_t bytes = plain_layout(num_taps, kFmt, T * R).bytes;
+        const cudaError_t e =
+            spread_tiles(reinterpret_cast<const void*>(kernel), tiles, sms, 1024 / T, &bytes);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        return launch_overlapped(kernel, static_cast<unsigned>(tiles), T, bytes, stream, x, taps,
+                                 static_cast<float2*>(y), n, num_taps);
+    });
 }
 
 cudaError_t fir_plain_launch(const void* x, const float* taps, void* y, long long n,
                              int num_taps, cudaStream_t stream)
 {
-    if (n <= 0) {
-        return cudaSuccess;
-    }
-    const long long tiles = (n + kTile - 1) / kTile;
-    size_t bytes = fir_plain_smem_bytes(num_taps);
-    const cudaError_t err =
-        spread_tiles(reinterpret_cast<const void*>(fir_plain_kernel), tiles, &bytes);
-    if (err != cudaSuccess) {
-        return err;
-    }
-    return launch_overlapped(fir_plain_kernel, static_cast<unsigned>(tiles), kThreads, bytes, stream,
-                             static_cast<const float2*>(x), taps, static_cast<float2*>(y), n,
-                             num_taps);
+    return launch_plain<0>(x, taps, y, n, num_taps, stream);
 }
 
 cudaError_t fir_plain_batched_launch(const PlainBatch& batch, int count, const float* taps,
                                      int num_taps, cudaStream_t stream)
 {
     long long longest = 0;
+    long long total = 0;
     for (int c = 0; c < count; ++c) {
         longest = batch.num_samples[c] > longest ? batch.num_samples[c] : longest;
+        total += batch.num_samples[c];
     }
     if (longest == 0) {
         return cudaSuccess;
     }
-    const dim3 grid(static_cast<unsigned>((longest + kTile - 1) / kTile), count);
-    size_t bytes = fir_plain_smem_bytes(num_taps);
-    const cudaError_t err =
-        spread_tiles(reinterpret_cast<const void*>(fir_plain_batched_kernel),
-                     static_cast<long long>(grid.x) * count, &bytes);
+    int sms = 0;
+    const cudaError_t err = sm_count(&sms);
     if (err != cudaSuccess) {
         return err;
     }
-    return launch_overlapped(fir_plain_batched_kernel, grid, kThreads, bytes, stream, batch, taps,
-                             num_taps);
+    return with_shape(tile_shape(total, num_taps, sms), [&](auto r, auto t) {
+        constexpr int R = decltype(r)::value;
+        constexpr int T = decltype(t)::value;
+        auto kernel = fir_plain_batched_kernel<R, T>;
+        const dim3 grid(static_cast<unsigned>((longest + T * R - 1) / (T * R)), count);
+        size_t bytes = plain_layout(num_taps, 0, T * R).bytes;
+        const cudaError_t e =
+            spread_tiles(reinterpret_cast<const void*>(kernel),
+                         (total + T * R - 1) / (T * R) + count, sms, 1024 / T, &bytes);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        return launch_overlapped(kernel, grid, T, bytes, stream, batch, taps, num_taps);
+    });
 }
 
 cudaError_t fir_plain_launch_format(int format, const void* x, const float* taps, void* y,
                                     long long n, int num_taps, cudaStream_t stream)
 {
-    if (format == 0) {
-        return fir_plain_launch(x, taps, y, n, num_taps, stream);
+    switch (format) {
+    case 1: return launch_plain<1>(x, taps, y, n, num_taps, stream);
+    case 2: return launch_plain<2>(x, taps, y, n, num_taps, stream);
+    default: return launch_plain<0>(x, taps, y, n, num_taps, stream);
     }
-    if (n <= 0) {
-        return cudaSuccess;
-    }
-    const long long tiles = (n + kTile - 1) / kTile;
-    size_t bytes = plain_layout(num_taps, format).bytes;
-    const void* fn = format == 1 ? reinterpret_cast<const void*>(fir_plain_fmt_kernel<1>)
-                                 : reinterpret_cast<const void*>(fir_plain_fmt_kernel<2>);
-    const cudaError_t err = spread_tiles(fn, tiles, &bytes);
-    if (err != cudaSuccess) {
-        return err;
-    }
-    return launch_overlapped(format == 1 ? fir_plain_fmt_kernel<1> : fir_plain_fmt_kernel<2>,
-                             static_cast<unsigned>(tiles), kThreads, bytes, stream, x, taps,
-                             static_cast<float2*>(y), n, num_taps);
 }
 
 cudaError_t fir_plain_caps_launch(const PlainCaps& caps, cudaStream_t stream)
@@ -201,9 +270,13 @@ cudaError_t fir_plain_caps_launch(const PlainCaps& caps, cudaStream_t stream)
     for (int c = 0; c < caps.count; ++c) {
         kmax = caps.num_taps[c] > kmax ? caps.num_taps[c] : kmax;
     }
-    size_t bytes = fir_plain_smem_bytes(kmax);
-    const cudaError_t err =
-        spread_tiles(reinterpret_cast<const void*>(fir_plain_caps_kernel), tiles, &bytes);
+    int sms = 0;
+    cudaError_t err = sm_count(&sms);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    size_t bytes = plain_layout(kmax).bytes;
+    err = spread_tiles(reinterpret_cast<const void*>(fir_plain_caps_kernel), tiles, sms, 4, &bytes);
     if (err != cudaSuccess) {
         return err;
     }

@@ -32,7 +32,6 @@ struct PlainCaps {
     int count;
 };
 
-size_t fir_plain_smem_bytes(int num_taps);
 cudaError_t fir_plain_launch(const void* x, const float* taps, void* y, long long n,
                              int num_taps, cudaStream_t stream);
 cudaError_t fir_plain_batched_launch(const PlainBatch& batch, int count, const float* taps,

@@ -4,6 +4,9 @@
 //
 //   y[n] = sum_{k=0}^{K-1} h[k] x[n-k],  x[m] = 0 for m < 0,  n < N      (src/fir.cu:1-5)
 //
+// Written for R outputs per thread and T threads; described at R = 9 and T = 256, what large
+// inputs run (fir_plain.cu has the rule).
+//
 // Arithmetic: every output is one chain of fused multiply-adds over k = 0, 1, ..., K-1 starting
 // from +0.0f, separately for I and Q. That is the order of the project's naive, tiled and
 // register kernels (src/fir.cu:35-40, :377-395), so the results are bit-identical to theirs.
@@ -63,14 +66,14 @@ struct Layout {
 // Bytes per sample of each input format (rfx_sample_format): cf32, ci16, ci8.
 __host__ __device__ constexpr uint32_t sample_bytes(int fmt) { return fmt == 0 ? 8u : fmt == 1 ? 4u : 2u; }
 
-__host__ __device__ inline Layout plain_layout(int num_taps, int fmt = 0)
+__host__ __device__ inline Layout plain_layout(int num_taps, int fmt = 0, int tile = kTile)
 {
     Layout l;
     l.taps_off = 16;
     l.tile_off = (l.taps_off + 8u * static_cast<uint32_t>(num_taps) + 15u) & ~15u;
-    const uint32_t tile_samples = kGuard + kTile + static_cast<uint32_t>(num_taps) + 8u;
+    const uint32_t tile_samples = kGuard + static_cast<uint32_t>(tile) + static_cast<uint32_t>(num_taps) + 8u;
     l.raw_off = (l.tile_off + 8u * tile_samples + 15u) & ~15u;
-    l.bytes = l.raw_off + (fmt == 0 ? 0u : sample_bytes(fmt) * (kTile + static_cast<uint32_t>(num_taps) + 8u));
+    l.bytes = l.raw_off + (fmt == 0 ? 0u : sample_bytes(fmt) * (static_cast<uint32_t>(tile) + static_cast<uint32_t>(num_taps) + 8u));
     return l;
 }
 
@@ -88,74 +91,94 @@ __device__ __forceinline__ f32x2 decode_sample(const void* raw, long long i)
     return pack2(static_cast<float>(v.x) * (1.0f / 128.0f), static_cast<float>(v.y) * (1.0f / 128.0f));
 }
 
-// Nine taps 9g + q (q < nq) against output window blocks: cur = S_g, nxt = S_{g+1}.
-__device__ __forceinline__ void tap_group(f32x2 (&acc)[kR], const f32x2 (&cur)[kR],
-                                          const f32x2 (&nxt)[kR], const f32x2* taps2, int k0,
+// R taps R g + q (q < nq) against output window blocks: cur = S_g, nxt = S_{g+1}.
+template <int R>
+__device__ __forceinline__ void tap_group(f32x2 (&acc)[R], const f32x2 (&cur)[R],
+                                          const f32x2 (&nxt)[R], const f32x2* taps2, int k0,
                                           int nq)
 {
 #pragma unroll
-    for (int q = 0; q < kR; ++q) {
+    for (int q = 0; q < R; ++q) {
         if (q < nq) {
             const f32x2 h = taps2[k0 + q];
 #pragma unroll
-            for (int j = 0; j < kR; ++j) {
-                acc[j] = fma2(h, j >= q ? cur[j - q] : nxt[kR + j - q], acc[j]);
+            for (int j = 0; j < R; ++j) {
+                acc[j] = fma2(h, j >= q ? cur[j - q] : nxt[R + j - q], acc[j]);
             }
         }
     }
 }
 
-__device__ __forceinline__ void load_block(f32x2 (&blk)[kR], const f32x2* tile, int p, int m)
+template <int R>
+__device__ __forceinline__ void load_block(f32x2 (&blk)[R], const f32x2* tile, int p, int m)
 {
-    // S_m[i] = x[n0 - 9m + i] = tile[p - 9m + i]
-    const f32x2* src = tile + (p - kR * m);
+    // S_m[i] = x[n0 - R m + i] = tile[p - R m + i]
+    const f32x2* src = tile + (p - R * m);
 #pragma unroll
-    for (int i = 0; i < kR; ++i) {
+    for (int i = 0; i < R; ++i) {
         blk[i] = src[i];
     }
 }
 
-// Computes this thread's nine outputs of the tile staged at `tile` (tile[i] = x[base + i]).
-__device__ __forceinline__ void compute_outputs(f32x2 (&acc)[kR], const f32x2* tile,
+// Computes this thread's R outputs of the tile staged at `tile` (tile[i] = x[base + i]).
+template <int R>
+__device__ __forceinline__ void compute_outputs(f32x2 (&acc)[R], const f32x2* tile,
                                                 const f32x2* taps2, int p, int num_taps)
 {
 #pragma unroll
-    for (int j = 0; j < kR; ++j) {
+    for (int j = 0; j < R; ++j) {
         acc[j] = 0ull;  // +0.0f, +0.0f
     }
-    const int groups = num_taps / kR;
-    const int rem = num_taps - groups * kR;
-    f32x2 a[kR];
-    f32x2 b[kR];
+    const int groups = num_taps / R;
+    const int rem = num_taps - groups * R;
+    f32x2 a[R];
+    f32x2 b[R];
     load_block(a, tile, p, 0);
     int g = 0;
     for (; g + 2 <= groups; g += 2) {
+        // 2 R taps from an even one on, two per 16-byte load.
         load_block(b, tile, p, g + 1);
-        tap_group(acc, a, b, taps2, kR * g, kR);
-        load_block(a, tile, p, g + 2);
-        tap_group(acc, b, a, taps2, kR * (g + 1), kR);
+        const ulonglong2* pair = reinterpret_cast<const ulonglong2*>(taps2 + R * g);
+        ulonglong2 h{};
+#pragma unroll
+        for (int t = 0; t < 2 * R; ++t) {
+            if (t == R) {
+                load_block(a, tile, p, g + 2);
+            }
+            if (t % 2 == 0) {
+                h = pair[t / 2];
+            }
+            const int q = t % R;
+            const f32x2 ht = t % 2 == 0 ? h.x : h.y;
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                const f32x2 v = t < R ? (j >= q ? a[j - q] : b[R + j - q])
+                                      : (j >= q ? b[j - q] : a[R + j - q]);
+                acc[j] = fma2(ht, v, acc[j]);
+            }
+        }
     }
     if (g < groups) {
         load_block(b, tile, p, g + 1);
-        tap_group(acc, a, b, taps2, kR * g, kR);
+        tap_group(acc, a, b, taps2, R * g, R);
         if (rem > 0) {
             load_block(a, tile, p, g + 2);
-            tap_group(acc, b, a, taps2, kR * (g + 1), rem);
+            tap_group(acc, b, a, taps2, R * (g + 1), rem);
         }
     } else if (rem > 0) {
         load_block(b, tile, p, g + 1);
-        tap_group(acc, a, b, taps2, kR * g, rem);
+        tap_group(acc, a, b, taps2, R * g, rem);
     }
 }
 
 }  // namespace plain
 
-// One tile of one capture, computed by the 256 threads tid = 0..255 of a group that synchronizes
-// with `sync`; the tile's mbarrier sits at smem offset 0 (initialized by this call if `init`,
+// One tile (T R outputs) of one capture, computed by the T threads tid = 0 .. T - 1 of a group that
+// synchronizes with `sync`; the tile's mbarrier sits at smem offset 0 (initialized by this call if `init`,
 // its expected phase in `phase`, advanced when the tile used it). Returns false if the tile's
 // copy did not arrive within the wait limit (recorded in *fault). kFmt: the input's sample
 // format (0 cf32; 1 ci16, 2 ci8: decoded into cf32 in shared memory).
-template <int kFmt = 0, class Sync = PlainBlockSync>
+template <int kFmt = 0, int R = plain::kR, int T = plain::kThreads, class Sync = PlainBlockSync>
 __device__ __forceinline__ bool fir_plain_tile(const void* __restrict__ xv,
                                                const float* __restrict__ taps,
                                                float2* __restrict__ y, long long n,
@@ -165,7 +188,9 @@ __device__ __forceinline__ bool fir_plain_tile(const void* __restrict__ xv,
 {
     using namespace plain;
     const float2* x = static_cast<const float2*>(xv);
-    const Layout lay = plain_layout(num_taps, kFmt);
+    constexpr int kTile = T * R;
+    static_assert(kTile % 2 == 0, "tiles start on 16-byte boundaries");
+    const Layout lay = plain_layout(num_taps, kFmt, kTile);
     const uint32_t sbase = smem_u32(smem);
     const uint32_t bar = sbase;  // mbarrier at offset 0
     f32x2* taps2 = reinterpret_cast<f32x2*>(smem + lay.taps_off);
@@ -195,7 +220,7 @@ __device__ __forceinline__ bool fir_plain_tile(const void* __restrict__ xv,
         }
     }
     // Taps (duplicated into both lanes) and the guard while the copy is in flight.
-    for (int k = tid; k < num_taps; k += kThreads) {
+    for (int k = tid; k < num_taps; k += T) {
         const float h = __ldg(taps + k);
         taps2[k] = pack2(h, h);
     }
@@ -203,7 +228,7 @@ __device__ __forceinline__ bool fir_plain_tile(const void* __restrict__ xv,
         guard[tid] = 0ull;
     }
     if (!interior) {
-        for (int i = tid; i < tile_len; i += kThreads) {
+        for (int i = tid; i < tile_len; i += T) {
             const long long m = base + i;
             f32x2 v = 0ull;
             if (m >= 0 && m < n) {
@@ -225,23 +250,23 @@ __device__ __forceinline__ bool fir_plain_tile(const void* __restrict__ xv,
         if (kFmt != 0) {
             // Decode the staged components into the sample tile.
             const unsigned char* raw = smem + lay.raw_off;
-            for (int i = tid; i < tile_len; i += kThreads) {
+            for (int i = tid; i < tile_len; i += T) {
                 tile[i] = decode_sample<kFmt>(raw, i);
             }
             sync();
         }
     }
 
-    const long long n0 = t0 + static_cast<long long>(kR) * tid;
-    f32x2 acc[kR];
+    const long long n0 = t0 + static_cast<long long>(R) * tid;
+    f32x2 acc[R];
     if (ok && n0 < n) {
         compute_outputs(acc, tile, taps2, static_cast<int>(n0 - base), num_taps);
     }
     sync();  // every thread is done reading the tile: reuse it for the results
     if (ok && n0 < n) {
 #pragma unroll
-        for (int j = 0; j < kR; ++j) {
-            tile[kR * tid + j] = acc[j];
+        for (int j = 0; j < R; ++j) {
+            tile[R * tid + j] = acc[j];
         }
     }
     if (interior) {
@@ -259,7 +284,7 @@ __device__ __forceinline__ bool fir_plain_tile(const void* __restrict__ xv,
         }
     } else {
         const long long valid = n - t0 < kTile ? n - t0 : kTile;
-        for (int i = tid; i < valid; i += kThreads) {
+        for (int i = tid; i < valid; i += T) {
             const float2 v = unpack2(tile[i]);
             y[t0 + i] = v;
         }
