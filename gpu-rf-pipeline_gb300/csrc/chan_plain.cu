@@ -12,11 +12,11 @@
 // s_d = x[dM - m] with taps g_p = h[pM + m], and consecutive threads take consecutive branches,
 // so every sample and tap load of a warp is one coalesced 256-byte row; the I/Q pair is one
 // packed f32x2 fused multiply-add. Two forms:
-//  - chan_branch_ring_kernel (8, 16, 24 or 32 taps in every branch): a thread walks one branch
-//    through a segment of frames keeping the window of its current 8 frames in registers, so
-//    each sample is loaded once (2^26 samples, 1024 channels, 32 taps per branch: 187 us under
+//  - chan_branch_ring_kernel (up to 32 taps per branch): a thread walks one branch through a
+//    segment of frames keeping the window of its current 8 frames in registers, so each sample is
+//    loaded once (2^26 samples, 1024 channels, 32 taps per branch: 187 us under
 //    the profiler, 84 % of the HBM copy rate, against 350 us for the form below);
-//  - chan_branch_kernel (any tap count): a thread computes R = 8 consecutive frames of one
+//  - chan_branch_kernel (more taps): a thread computes R = 8 consecutive frames of one
 //    branch with two alternating 8-sample register blocks, so each sample is loaded
 //    (R + P - 1) / R times instead of P times.
 // Frame groups whose terms fall before the input, and the last group (past its end), take a
@@ -27,6 +27,8 @@
 
 #include <cuda_runtime.h>
 #include <cufft.h>
+
+#include <type_traits>
 
 namespace rfx {
 
@@ -190,18 +192,28 @@ chan_branch_kernel(const void* __restrict__ x, const float* __restrict__ taps,
     }
 }
 
-// Register-ring form, for filters of exactly 8, 16, 24 or 32 taps in every branch (num_taps =
-// P * channels; cf32 and ci16 input). A thread owns one branch m and one segment of
-// consecutive frames, which it walks in steps of kR = 8 frames. The samples of its branch for
-// the current step and the P / 8 steps before it (a step's window: P + 8 decimated samples)
-// stay in registers as P / 8 + 1 blocks of eight, so every sample is loaded once per segment
-// instead of once per tap group, and the branch's taps stay in registers too. The next blocks
-// stream in by per-thread asynchronous copies, kRingStages steps ahead, into the thread's own
-// slots of a shared-memory stage ring (a warp's copies and reads of one block row are 256
-// contiguous bytes). Terms are summed in branch_frames' order: taps ascending from +0, one
-// fused multiply-add each; steps whose terms reach before the input (t0 < guard_frames) take
-// branch_frames' tested path. Every branch having all P taps, the tap loop has no per-branch
-// test (measured: a per-tap test of the branch's tap count doubled the instructions issued).
+// Register-ring form, for filters of up to 32 taps per branch. A thread owns one branch m and one
+// segment of consecutive frames, which it walks in steps of kR = 8 frames. The samples of its
+// branch for the current step and the kPG steps before it (kPG tap groups of eight) stay in
+// registers as kPG + 1 blocks of eight, so every sample is loaded once per segment instead of once
+// per tap group, and the branch's taps stay in registers too. The next blocks stream in by
+// per-thread asynchronous copies, kRingStages steps ahead, into the thread's own slots of a
+// shared-memory stage ring (a warp's copies and reads of one block row are 256 contiguous bytes);
+// ci8 samples, narrower than such a copy, are loaded one step ahead into registers. Terms are
+// summed in branch_frames' order: taps ascending from +0, one fused multiply-add each, absent
+// taps and samples before the input left out.
+// Three forms of the step (Ring), which differ in the tests around the tap loop:
+//  * kLong: 8 kPG taps in every branch, long segments. No test in the loop (a per-tap test of the
+//    branch's tap count doubled the instructions issued); the segment that starts the input sums
+//    its first frames with branch_frames' tested path, from global memory.
+//  * kUniform: the same taps, short segments. The first frames too come from the window, each term
+//    tested, in a second copy of the loop: 1024 channels, 32 taps, sums and transform (us): 2^20
+//    samples 15.3 against 18.5 for kLong, 2^22 39.5 against 41.1, but 2^26 389 against 348 (the
+//    longer step code falls out of the instruction cache).
+//  * kAny: any tap count, any format; the last tap group tests the branch's tap count as well, and
+//    beyond 16 taps the window moves on one block per step instead of the code being repeated per
+//    position (32763 taps, 2^22 samples: 41.7 us against 80). Against chan_branch_kernel, which
+//    took these filters: 2^20 samples, 12287 taps 12.9 against 28.7, 32763 taps 22.4 against 52.2.
 constexpr int kRingThreads = 128;
 constexpr int kRingStages = 4;
 
@@ -218,17 +230,29 @@ __device__ __forceinline__ f32x2 ring_lds(uint32_t addr)
     }
 }
 
-template <int kPG, int kFmt>
-__global__ void __launch_bounds__(kRingThreads, 3)
+// Blocks per SM: what the registers of the window and the taps leave.
+__host__ __device__ constexpr int ring_blocks(int groups)
+{
+    return groups == 1 ? 5 : groups == 2 ? 4 : 3;
+}
+
+enum class Ring { kLong, kUniform, kAny };
+
+template <int kPG, int kFmt, Ring kRing>
+__global__ void __launch_bounds__(kRingThreads, ring_blocks(kPG))
 chan_branch_ring_kernel(const void* __restrict__ x, const float* __restrict__ taps,
                         float2* __restrict__ u, long long n, long long frames, int channels,
-                        int width, long long seg_frames, int guard_frames)
+                        int num_taps, int width, long long seg_frames, int guard_frames)
 {
     constexpr int kN = kPG + 1;                  // register blocks
     constexpr int kP = kR * kPG;                 // taps per branch
-    constexpr int kSb = kFmt == 0 ? 8 : 4;       // bytes per stored sample
+    constexpr int kSb = kFmt == 0 ? 8 : kFmt == 1 ? 4 : 2;       // bytes per stored sample
+    constexpr bool kCopies = kFmt != 2;
+    constexpr bool kGeneral = kRing == Ring::kAny;
+    constexpr bool kGuard = kRing != Ring::kLong;    // the first frames from the window too
+    constexpr bool kRotate = !kGeneral || kPG <= 2;   // else the window moves on one block per step
     constexpr uint32_t kStageBytes = kR * kRingThreads * kSb;
-    __shared__ __align__(16) unsigned char stage[kRingStages * kStageBytes];
+    __shared__ __align__(16) unsigned char stage[kCopies ? kRingStages * kStageBytes : 16];
     wait_for_stream();
     allow_next();
     const int tid = static_cast<int>(threadIdx.x);
@@ -243,34 +267,41 @@ chan_branch_ring_kernel(const void* __restrict__ x, const float* __restrict__ ta
     float g[kP];
 #pragma unroll
     for (int p = 0; p < kP; ++p) {
-        g[p] = __ldg(taps + static_cast<long long>(p) * channels + m);
+        const long long l = static_cast<long long>(p) * channels + m;
+        g[p] = !kGeneral || l < num_taps ? __ldg(taps + l) : 0.0f;
     }
+    const int my_taps = m < num_taps ? (num_taps - m + channels - 1) / channels : 0;
+    const bool full = num_taps == kP * channels;
+    const long long first_valid = m > 0 ? 1 : 0;   // x[dM - m] lies in the input from this d on
     long long t0 = f0;
-    for (; t0 < f1 && t0 < guard_frames; t0 += kR) {
-        f32x2 acc[kR];
+    if constexpr (!kGuard) {
+        for (; t0 < f1 && t0 < guard_frames; t0 += kR) {
+            f32x2 acc[kR];
 #pragma unroll
-        for (int i = 0; i < kR; ++i) {
-            acc[i] = 0ull;
-        }
-        branch_frames<true, kFmt>(acc, x, taps + m, channels, n, channels, m, kP, t0);
+            for (int i = 0; i < kR; ++i) {
+                acc[i] = 0ull;
+            }
+            branch_frames<true, kFmt>(acc, x, taps + m, channels, n, channels, m, kP, t0);
 #pragma unroll
-        for (int i = 0; i < kR; ++i) {
-            if (t0 + i < f1) {
-                u[(t0 + i) * channels + m] = unpack2(acc[i]);
+            for (int i = 0; i < kR; ++i) {
+                if (t0 + i < f1) {
+                    u[(t0 + i) * channels + m] = unpack2(acc[i]);
+                }
             }
         }
-    }
-    if (t0 >= f1) {
-        return;
+        if (t0 >= f1) {
+            return;
+        }
     }
     // Ring slot k % kN holds block B(t0 + 8k) (decimated samples t0 + 8k .. + 7) during step k;
-    // the blocks before step 0 go to slots kN - q, q = 1 .. kPG (all at indices >= 8 M - m).
+    // the blocks before step 0 go to slots kN - q, q = 1 .. kPG (zeros before the input).
     f32x2 R[kN][kR];
 #pragma unroll
     for (int q = 1; q <= kPG; ++q) {
 #pragma unroll
         for (int i = 0; i < kR; ++i) {
-            R[kN - q][i] = load_sample<kFmt>(x, (t0 - kR * q + i) * channels - m);
+            const long long s = (t0 - kR * q + i) * channels - m;
+            R[kN - q][i] = s >= 0 ? load_sample<kFmt>(x, s) : 0ull;
         }
     }
     // Sample d of the branch is at byte (d M - m) kSb of x: consecutive d are `row` bytes apart.
@@ -282,10 +313,24 @@ chan_branch_ring_kernel(const void* __restrict__ x, const float* __restrict__ ta
     // the segment.
     const char* src = static_cast<const char*>(x) + (t0 * channels - m) * kSb;
     long long src_left = f1 - t0;
+    bool src_first = t0 == 0;   // its frame 0 reads x[-m] in all branches but the first
     uint32_t src_stage = 0;
+    unsigned short pre[kCopies ? 1 : kR];   // ci8: the next step's samples
     auto issue = [&]() {
+        if constexpr (!kCopies) {
+#pragma unroll
+            for (int i = 0; i < kR; ++i) {
+                const bool ok = i < src_left && (i > 0 || !src_first || m == 0);
+                pre[i] = ok ? __ldg(reinterpret_cast<const unsigned short*>(src + i * row))
+                            : static_cast<unsigned short>(0);
+            }
+            src += kR * row;
+            src_left -= kR;
+            src_first = false;
+            return;
+        }
         const uint32_t dst = sbase + src_stage * kStageBytes;
-        if (src_left >= kR) {
+        if (src_left >= kR && !src_first) {
             const char* s = src;
 #pragma unroll
             for (int i = 0; i < kR; ++i) {
@@ -296,37 +341,53 @@ chan_branch_ring_kernel(const void* __restrict__ x, const float* __restrict__ ta
             const char* s = src;
 #pragma unroll
             for (int i = 0; i < kR; ++i) {
-                const bool ok = i < src_left;
-                cp_async<kSb>(dst + static_cast<uint32_t>(i * kRingThreads * kSb), ok ? s : src,
-                              ok ? kSb : 0);
+                const bool ok = i < src_left && (i > 0 || !src_first || m == 0);
+                cp_async<kSb>(dst + static_cast<uint32_t>(i * kRingThreads * kSb),
+                              ok ? s : static_cast<const char*>(x), ok ? kSb : 0);
                 s += row;
             }
         }
         cp_async_commit();
         src += kR * row;
         src_left -= kR;
+        src_first = false;
         src_stage = src_stage + 1 == kRingStages ? 0 : src_stage + 1;
     };
 #pragma unroll
-    for (int s = 0; s < kRingStages - 1; ++s) {
+    for (int s = 0; s < (kCopies ? kRingStages - 1 : 1); ++s) {
         issue();
     }
     float2* dst = u + t0 * channels + m;
     long long dst_left = f1 - t0;
     uint32_t read_stage = 0;
-    for (long long k0 = 0; k0 < nb; k0 += kN) {
+    constexpr int kRots = kRotate ? kN : 1;
+    for (long long k0 = 0; k0 < nb; k0 += kRots) {
 #pragma unroll
-        for (int rot = 0; rot < kN; ++rot) {
+        for (int rot = 0; rot < kRots; ++rot) {
             if (k0 + rot < nb) {
-                // Refills the stage read in the step before with the block kRingStages - 1
-                // steps ahead, then waits for this step's block.
-                issue();
-                cp_async_wait<kRingStages - 1>();
-                const uint32_t rs = sbase + read_stage * kStageBytes;
-                read_stage = read_stage + 1 == kRingStages ? 0 : read_stage + 1;
+                if constexpr (kCopies) {
+                    // Refills the stage read in the step before with the block kRingStages - 1
+                    // steps ahead, then waits for this step's block.
+                    issue();
+                    cp_async_wait<kRingStages - 1>();
+                    const uint32_t rs = sbase + read_stage * kStageBytes;
+                    read_stage = read_stage + 1 == kRingStages ? 0 : read_stage + 1;
 #pragma unroll
-                for (int i = 0; i < kR; ++i) {
-                    R[rot][i] = ring_lds<kFmt>(rs + static_cast<uint32_t>(i * kRingThreads * kSb));
+                    for (int i = 0; i < kR; ++i) {
+                        R[rot][i] =
+                            ring_lds<kFmt>(rs + static_cast<uint32_t>(i * kRingThreads * kSb));
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kR; ++i) {
+                        const int v = pre[i];
+                        R[rot][i] = pack2(
+                            static_cast<float>(static_cast<int>(static_cast<uint32_t>(v) << 24) >> 24) *
+                                (1.0f / 128.0f),
+                            static_cast<float>(static_cast<int>(static_cast<uint32_t>(v) << 16) >> 24) *
+                                (1.0f / 128.0f));
+                    }
+                    issue();
                 }
                 f32x2 acc[kR];
 #pragma unroll
@@ -334,16 +395,40 @@ chan_branch_ring_kernel(const void* __restrict__ x, const float* __restrict__ ta
                     acc[i] = 0ull;
                 }
                 // Tap group gq: cur = B(T - 8 gq), nxt = B(T - 8 gq - 8), T = t0 + 8 k.
+                const long long T = t0 + kR * (k0 + rot);
 #pragma unroll
                 for (int gq = 0; gq < kPG; ++gq) {
                     const int cs = (rot - gq + 2 * kN) % kN;
                     const int ns = (rot - gq - 1 + 2 * kN) % kN;
-#pragma unroll
-                    for (int q = 0; q < kR; ++q) {
+                    auto tap = [&](int q, auto guarded) {
                         const f32x2 h2 = pack2(g[kR * gq + q], g[kR * gq + q]);
 #pragma unroll
                         for (int i = 0; i < kR; ++i) {
-                            acc[i] = fma2(h2, i >= q ? R[cs][i - q] : R[ns][kR + i - q], acc[i]);
+                            if (!decltype(guarded)::value ||
+                                T + i - (kR * gq + q) >= first_valid) {
+                                acc[i] = fma2(h2, i >= q ? R[cs][i - q] : R[ns][kR + i - q],
+                                              acc[i]);
+                            }
+                        }
+                    };
+                    if (kGuard && T < guard_frames) {
+#pragma unroll
+                        for (int q = 0; q < kR; ++q) {
+                            if (!kGeneral || kR * gq + q < my_taps) {
+                                tap(q, std::true_type{});
+                            }
+                        }
+                    } else if (!kGeneral || gq < kPG - 1 || full) {
+#pragma unroll
+                        for (int q = 0; q < kR; ++q) {
+                            tap(q, std::false_type{});
+                        }
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < kR; ++q) {
+                            if (kR * gq + q < my_taps) {
+                                tap(q, std::false_type{});
+                            }
                         }
                     }
                 }
@@ -366,37 +451,57 @@ chan_branch_ring_kernel(const void* __restrict__ x, const float* __restrict__ ta
                 }
                 dst += static_cast<long long>(kR) * channels;
                 dst_left -= kR;
+                if constexpr (!kRotate) {
+                    // Every block one place older.
+#pragma unroll
+                    for (int q = 1; q < kN; ++q) {
+#pragma unroll
+                        for (int i = 0; i < kR; ++i) {
+                            R[q][i] = R[(q + 1) % kN][i];
+                        }
+                    }
+                }
             }
         }
     }
-    cp_async_wait<0>();
+    if constexpr (kCopies) {
+        cp_async_wait<0>();
+    }
+}
+
+using RingKernel = void (*)(const void*, const float*, float2*, long long, long long, int, int, int,
+                            long long, int);
+
+template <int kFmt, Ring kRing>
+static RingKernel ring_kernel(int groups)
+{
+    switch (groups) {
+    case 1: return chan_branch_ring_kernel<1, kFmt, kRing>;
+    case 2: return chan_branch_ring_kernel<2, kFmt, kRing>;
+    case 3: return chan_branch_ring_kernel<3, kFmt, kRing>;
+    default: return chan_branch_ring_kernel<4, kFmt, kRing>;
+    }
+}
+
+template <int kFmt>
+static RingKernel ring_kernel(int groups, Ring ring)
+{
+    return ring == Ring::kLong      ? ring_kernel<kFmt, Ring::kLong>(groups)
+           : ring == Ring::kUniform ? ring_kernel<kFmt, Ring::kUniform>(groups)
+                                    : ring_kernel<kFmt, Ring::kAny>(groups);
 }
 
 static cudaError_t ring_launch(const void* x, const float* taps, float2* u, long long n,
-                               long long frames, int channels, int per_branch,
-                               cudaStream_t stream, int format)
+                               long long frames, int channels, int num_taps, cudaStream_t stream,
+                               int format)
 {
-    void (*fn)(const void*, const float*, float2*, long long, long long, int, int, long long, int) =
-        nullptr;
-    switch (per_branch / kR * 2 + format) {
-    case 2: fn = chan_branch_ring_kernel<1, 0>; break;
-    case 3: fn = chan_branch_ring_kernel<1, 1>; break;
-    case 4: fn = chan_branch_ring_kernel<2, 0>; break;
-    case 5: fn = chan_branch_ring_kernel<2, 1>; break;
-    case 6: fn = chan_branch_ring_kernel<3, 0>; break;
-    case 7: fn = chan_branch_ring_kernel<3, 1>; break;
-    case 8: fn = chan_branch_ring_kernel<4, 0>; break;
-    case 9: fn = chan_branch_ring_kernel<4, 1>; break;
-    default: return cudaErrorInvalidValue;
-    }
+    const int groups = static_cast<int>((num_taps + static_cast<long long>(kR) * channels - 1) /
+                                        (static_cast<long long>(kR) * channels));
     int device = 0;
     int sms = 0;
-    int occ = 0;
     cudaError_t err = cudaGetDevice(&device);
     if (err != cudaSuccess ||
         (err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) !=
-            cudaSuccess ||
-        (err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kRingThreads, 0)) !=
             cudaSuccess) {
         return err;
     }
@@ -408,23 +513,27 @@ static cudaError_t ring_launch(const void* x, const float* taps, float2* u, long
     }
     const int per_block = kRingThreads / w;
     const long long gy = (channels + w - 1) / w;
-    const long long capacity = static_cast<long long>(sms) * (occ > 0 ? occ : 1);
+    const long long capacity = static_cast<long long>(sms) * ring_blocks(groups);
     const long long bx_target = capacity / gy > 0 ? capacity / gy : 1;
     const long long segs_target = bx_target * per_block;
     long long seg_frames = (frames + segs_target - 1) / segs_target;
     seg_frames = (seg_frames + kR - 1) / kR * kR;
-    if (seg_frames < 8 * kR) {
-        seg_frames = 8 * kR;
-    }
     const long long segs = (frames + seg_frames - 1) / seg_frames;
     const long long bx = (segs + per_block - 1) / per_block;
     if (bx > 0x7FFFFFFFLL || gy > 65535) {
         return cudaErrorInvalidConfiguration;
     }
-    int guard_frames = kR * (per_branch / kR + 1);
+    const int guard_frames = kR * (groups + 1);
+    const long long long_segment = groups == 4 ? 160 : 256;
+    const Ring ring = num_taps != kR * groups * channels ? Ring::kAny
+                      : seg_frames < long_segment        ? Ring::kUniform
+                                                         : Ring::kLong;
+    const RingKernel fn = format == 2   ? ring_kernel<2, Ring::kAny>(groups)
+                          : format == 1 ? ring_kernel<1>(groups, ring)
+                                        : ring_kernel<0>(groups, ring);
     const dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(gy));
-    return launch_overlapped(fn, grid, kRingThreads, 0, stream, x, taps, u, n, frames, channels, w,
-                             seg_frames, guard_frames);
+    return launch_overlapped(fn, grid, kRingThreads, 0, stream, x, taps, u, n, frames, channels,
+                             num_taps, w, seg_frames, guard_frames);
 }
 
 cudaError_t chan_branch_launch(const void* x, const float* taps, void* u, long long frames,
@@ -435,10 +544,8 @@ cudaError_t chan_branch_launch(const void* x, const float* taps, void* u, long l
     }
     {
         const long long n = (frames - 1) * static_cast<long long>(channels) + 1;
-        const int per_branch = num_taps / channels;
-        if (format <= 1 && num_taps % channels == 0 && per_branch % kR == 0 &&
-            per_branch >= kR && per_branch <= 4 * kR) {
-            return ring_launch(x, taps, static_cast<float2*>(u), n, frames, channels, per_branch,
+        if (num_taps <= 4LL * kR * channels) {
+            return ring_launch(x, taps, static_cast<float2*>(u), n, frames, channels, num_taps,
                                stream, format);
         }
     }

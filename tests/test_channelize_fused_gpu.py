@@ -35,7 +35,7 @@ def inputs(n: int, k: int, seed: int) -> tuple[np.ndarray, np.ndarray]:
     return x, (rng.standard_normal(k) / np.sqrt(k)).astype(np.float32)
 
 
-@pytest.mark.parametrize("m", [16, 32, 64, 128, 256, 512])
+@pytest.mark.parametrize("m", [8, 16, 32, 64, 128, 256, 512])
 @pytest.mark.parametrize("blocks,more", [(0, 1), (1, -1), (1, 0), (7, 0), (8, 0), (8, 1), (15, 3),
                                          (16, 0), (17, 0), (24, 0), (25, -1), (31, 5), (32, 0)])
 def test_fused_matches_oracle(m: int, blocks: int, more: int) -> None:
@@ -99,3 +99,36 @@ def test_auto_at_64_channels_keeps_the_tensor_core_plans_limits() -> None:
         with pytest.raises(rfx.RfxError):
             plan.launch(dev(x), dev(h), out, num_samples=63)
     assert orc.normwise_error(want.cpu().numpy(), orc.channelize_fast(x, h, 64)) <= NORMWISE
+
+
+@pytest.mark.parametrize("m", [3, 100, 1000, 1024])
+@pytest.mark.parametrize("blocks,more", [(0, 1), (1, -1), (7, 2), (8, 0), (9, 0), (16, 0), (16, 1),
+                                         (23, -1), (24, 0), (25, 0), (31, 1), (32, 0)])
+def test_branch_sums_at_every_tap_count_keep_the_bits(m: int, blocks: int, more: int) -> None:
+    # The ring kernel's forms: uniform and partial last tap groups, inputs within the history, short
+    # segments, and (three channels) segments long enough for the form of long captures.
+    k = max(1, blocks * m + more)
+    for n in (1, 5 * m + 1, 60 * m + m // 2, (1 << 20) + 7 if m < 1000 else 400 * m + 9):
+        x, h = inputs(n, k, n + k)
+        u = rfx.channelize_branches(dev(x), dev(h), m)
+        want = orc.channelize_branch_f32_seq(x, h, m)
+        assert np.array_equal(bits(u), want.reshape(-1).view(np.uint32)), (n, k)
+
+
+@pytest.mark.parametrize("m,k", [(100, 1600), (100, 3101), (1024, 8192), (1024, 32768),
+                                 (1024, 12287), (8, 64), (8, 100)])
+@pytest.mark.parametrize("fmt", ["ci16", "ci8"])
+def test_ring_and_wide_formats_and_magnitude(m: int, k: int, fmt: str) -> None:
+    test_fused_formats_and_magnitude_bits(m, k, fmt)
+
+
+# The 1024-point transform, and where complex output goes over to cuFFT (8192 frames).
+@pytest.mark.parametrize("frames", [1, 3, 4, 5, 607, 609, 8192, 8193])
+def test_1024_channels_transform_matches_oracle(frames: int) -> None:
+    n, k = frames * 1024 - 7, 4096
+    x, h = inputs(n, k, frames)
+    z = rfx.channelize(dev(x), dev(h), 1024)
+    mag = rfx.channelize_magnitude(dev(x), dev(h), 1024)
+    ref = orc.channelize_fast(x, h, 1024)
+    assert orc.normwise_error(z.cpu().numpy(), ref) <= NORMWISE
+    assert np.max(np.abs(mag.cpu().numpy() - np.abs(ref))) <= NORMWISE * np.max(np.abs(ref))
