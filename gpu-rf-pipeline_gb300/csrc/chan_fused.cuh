@@ -1,4 +1,4 @@
-// Fused channelizer for M = 16, 32, ..., 512 channels and up to 32 taps per branch: polyphase
+// Fused channelizer for M = 8, 16, ..., 512 channels and up to 32 taps per branch: polyphase
 // branch sums and the M-point inverse transform in one pass over memory, in FP32.
 //
 //   u[t][m] = sum_p h[pM + m] x[tM - pM - m]           (x[i < 0] = 0)      src/channelize.cu:25-49
@@ -26,6 +26,7 @@
 // of the transform already keep the load/store pipe half busy.
 #pragma once
 
+#include "fft_small.cuh"
 #include "launch.hpp"
 #include "magnitude.cuh"
 #include "ptx.cuh"
@@ -38,157 +39,21 @@
 namespace rfx {
 namespace fused {
 
+using fft::cmul;
+using fft::small_dft;
+
 constexpr int kR = 8;                  // frames per step
 constexpr int kMaxGroups = 4;          // tap groups of eight per branch
 constexpr int kTablePoints = 512;      // e^{2 pi i k / 512}: every M divides it
 
-// The transform's roots of unity, rounded once from double. Built at compile time: sine and
-// cosine by their Taylor series on [0, pi / 4], the other octants by symmetry.
-struct Roots {
-    float v[2 * kTablePoints];
-};
-
-constexpr double taylor(double a, bool cosine)
-{
-    double term = cosine ? 1.0 : a;
-    double sum = term;
-    for (int k = cosine ? 1 : 2; k < 30; k += 2) {
-        term *= -a * a / (static_cast<double>(k) * (k + 1));
-        sum += term;
-    }
-    return sum;
-}
-
-constexpr Roots make_roots()
-{
-    Roots r{};
-    constexpr double kPi = 3.14159265358979323846264338327950288;
-    constexpr int kOctant = kTablePoints / 8;
-    for (int k = 0; k < kTablePoints; ++k) {
-        const int oct = k / kOctant;
-        const int rem = k % kOctant;
-        // Angle within the octant, mirrored in odd octants.
-        const double a = 2.0 * kPi * ((oct & 1) ? kOctant - rem : rem) / kTablePoints;
-        const double c = taylor(a, true);
-        const double s = taylor(a, false);
-        double re = 0.0;
-        double im = 0.0;
-        switch (oct) {
-        case 0: re = c; im = s; break;
-        case 1: re = s; im = c; break;
-        case 2: re = -s; im = c; break;
-        case 3: re = -c; im = s; break;
-        case 4: re = -c; im = -s; break;
-        case 5: re = -s; im = -c; break;
-        case 6: re = s; im = -c; break;
-        default: re = c; im = -s; break;
-        }
-        r.v[2 * k] = static_cast<float>(re);
-        r.v[2 * k + 1] = static_cast<float>(im);
-    }
-    return r;
-}
-
-// ---- small transforms in registers (inverse: w = e^{+2 pi i / r}) -----------------------------
-
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
-{
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
-{
-    f32x2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
-// a + i b and a - i b.
-__device__ __forceinline__ f32x2 add_i(f32x2 a, f32x2 b)
-{
-    const float2 p = unpack2(a);
-    const float2 q = unpack2(b);
-    return pack2(p.x - q.y, p.y + q.x);
-}
-
-__device__ __forceinline__ f32x2 sub_i(f32x2 a, f32x2 b)
-{
-    const float2 p = unpack2(a);
-    const float2 q = unpack2(b);
-    return pack2(p.x + q.y, p.y - q.x);
-}
-
-__device__ __forceinline__ f32x2 cmul(f32x2 a, float2 w)
-{
-    const float2 p = unpack2(a);
-    return pack2(__fmaf_rn(p.x, w.x, -__fmul_rn(p.y, w.y)),
-                 __fmaf_rn(p.x, w.y, __fmul_rn(p.y, w.x)));
-}
-
-template <int r>
-__device__ __forceinline__ void small_dft(f32x2* v)
-{
-    if constexpr (r == 2) {
-        const f32x2 a = v[0];
-        v[0] = add2(a, v[1]);
-        v[1] = sub2(a, v[1]);
-    } else if constexpr (r == 4) {
-        const f32x2 s0 = add2(v[0], v[2]);
-        const f32x2 d0 = sub2(v[0], v[2]);
-        const f32x2 s1 = add2(v[1], v[3]);
-        const f32x2 d1 = sub2(v[1], v[3]);
-        v[0] = add2(s0, s1);
-        v[1] = add_i(d0, d1);
-        v[2] = sub2(s0, s1);
-        v[3] = sub_i(d0, d1);
-    } else {
-        static_assert(r == 8, "radix 2, 4 or 8");
-        constexpr float c = 0.70710678118654752440f;
-        const f32x2 s0 = add2(v[0], v[4]);
-        const f32x2 d0 = sub2(v[0], v[4]);
-        const f32x2 s1 = add2(v[1], v[5]);
-        const f32x2 d1 = sub2(v[1], v[5]);
-        const f32x2 s2 = add2(v[2], v[6]);
-        const f32x2 d2 = sub2(v[2], v[6]);
-        const f32x2 s3 = add2(v[3], v[7]);
-        const f32x2 d3 = sub2(v[3], v[7]);
-        // Even outputs: the 4-point transform of s.
-        const f32x2 e0 = add2(s0, s2);
-        const f32x2 e1 = sub2(s0, s2);
-        const f32x2 e2 = add2(s1, s3);
-        const f32x2 e3 = sub2(s1, s3);
-        v[0] = add2(e0, e2);
-        v[4] = sub2(e0, e2);
-        v[2] = add_i(e1, e3);
-        v[6] = sub_i(e1, e3);
-        // Odd outputs: w8 d1 = c (1 + i) d1 and w8^3 d3 = c (-1 + i) d3.
-        const f32x2 f0 = add_i(d0, d2);
-        const f32x2 f1 = sub_i(d0, d2);
-        const float2 p = unpack2(d1);
-        const float2 q = unpack2(d3);
-        const f32x2 g1 = pack2(p.x - p.y, p.y + p.x);
-        const f32x2 g3 = pack2(-q.x - q.y, q.x - q.y);
-        const f32x2 h0 = add2(g1, g3);
-        const f32x2 h1 = sub2(g1, g3);
-        const f32x2 cc = pack2(c, c);
-        const f32x2 nc = pack2(-c, -c);
-        v[1] = fma2(cc, h0, f0);
-        v[5] = fma2(nc, h0, f0);
-        const float2 a = unpack2(f1);
-        const float2 b = unpack2(h1);
-        v[3] = pack2(__fmaf_rn(-c, b.y, a.x), __fmaf_rn(c, b.x, a.y));
-        v[7] = pack2(__fmaf_rn(c, b.y, a.x), __fmaf_rn(-c, b.x, a.y));
-    }
-}
-
 // ---- geometry ---------------------------------------------------------------------------------
 
 // Radices of the M-point transform, first to last (0: no such stage). The last radix leaves at
-// least eight consecutive channels per frame to eight consecutive lanes (64-byte stores).
+// least eight consecutive channels per frame to eight consecutive lanes (64-byte stores; four at
+// eight channels).
 template <int M>
 struct Radices;
+template <> struct Radices<8> { static constexpr int r[3] = {4, 2, 0}; };
 template <> struct Radices<16> { static constexpr int r[3] = {8, 2, 0}; };
 template <> struct Radices<32> { static constexpr int r[3] = {8, 4, 0}; };
 template <> struct Radices<64> { static constexpr int r[3] = {8, 8, 0}; };
@@ -348,7 +213,7 @@ __device__ __forceinline__ f32x2 decode(f32x2 raw)
     }
 }
 
-static __device__ const Roots kRootTable = make_roots();
+static __device__ const fft::Roots<kTablePoints> kRootTable = fft::make_roots<kTablePoints>();
 
 // kFmt: sample format of x (0 cf32, 1 ci16, 2 ci8). n: one past the newest sample any frame
 // reads. seg_frames: frames per segment, a multiple of eight. guard_frames: frames before it have

@@ -5,11 +5,11 @@
 
 namespace rfx {
 
-// Whether the fused kernel takes this shape: 16, 32, ..., 512 channels, at most 32 taps in any
+// Whether the fused kernel takes this shape: 8, 16, ..., 512 channels, at most 32 taps in any
 // branch.
 inline bool chan_fused_supported(int channels, int num_taps)
 {
-    return channels >= 16 && channels <= 512 && (channels & (channels - 1)) == 0 &&
+    return channels >= 8 && channels <= 512 && (channels & (channels - 1)) == 0 &&
            num_taps >= 1 && num_taps <= 32 * channels;
 }
 
@@ -17,6 +17,7 @@ inline bool chan_fused_supported(int channels, int num_taps)
     cudaError_t chan_fused_launch_##M(const void* x, const float* taps, void* out,                 \
                                       long long frames, int num_taps, bool magnitude, int format,  \
                                       cudaStream_t stream);
+RFX_CHAN_FUSED(8)
 RFX_CHAN_FUSED(16)
 RFX_CHAN_FUSED(32)
 RFX_CHAN_FUSED(64)
@@ -35,6 +36,7 @@ inline cudaError_t chan_fused_launch(const void* x, const float* taps, void* out
         return cudaSuccess;
     }
     switch (channels) {
+    case 8: return chan_fused_launch_8(x, taps, out, frames, num_taps, magnitude, format, stream);
     case 16: return chan_fused_launch_16(x, taps, out, frames, num_taps, magnitude, format, stream);
     case 32: return chan_fused_launch_32(x, taps, out, frames, num_taps, magnitude, format, stream);
     case 64: return chan_fused_launch_64(x, taps, out, frames, num_taps, magnitude, format, stream);

@@ -40,8 +40,8 @@ cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, 
 inline size_t even_spread_smem(size_t bytes, long long blocks, int sms, int fit)
 {
     const long long share = (blocks + sms - 1) / sms;
-    if (share >= fit) {
-        return bytes;
+    if (share >= fit || 2 * blocks <= sms) {
+        return bytes;   // a full wave, or few enough that idle multiprocessors remain
     }
     constexpr size_t kPerSm = 228u * 1024u;    // shared memory of an SM
     constexpr size_t kPerBlock = 1024u;        // of which the system takes this much per block

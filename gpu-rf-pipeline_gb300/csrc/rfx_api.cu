@@ -4,6 +4,7 @@
 
 #include "api_error.hpp"
 
+#include "chan_fft1024.hpp"
 #include "chan_fused.hpp"
 #include "chan_plain.cuh"
 #include "chan_tc.cuh"
@@ -609,7 +610,7 @@ int rfx_chan_plan_create(int impl, int channels, int64_t max_samples, rfx_chan_p
         *plan = p;
         return RFX_OK;
     }
-    if (p->frames > 0) {
+    if (p->frames > 0 && !(channels == 1024 && p->frames <= rfx::kFft1024Frames)) {
         int nfft = channels;
         const cufftResult r = cufftPlanMany(&p->fft, 1, &nfft, nullptr, 1, nfft, nullptr, 1,
                                             nfft, CUFFT_C2C, static_cast<int>(p->frames));
@@ -770,6 +771,14 @@ int channelize_plan(rfx_chan_plan* plan, const void* x, const float* taps, void*
             }
         }
         z = plan->scratch;
+    }
+    if (plan->channels == 1024 && (magnitude || !plan->has_fft)) {
+        cudaError_t err =
+            rfx::chan_branch_launch(x, taps, z, frames, plan->channels, num_taps, stream, format);
+        if (err == cudaSuccess) {
+            err = rfx::chan_fft1024_launch(z, out, frames, magnitude, stream);
+        }
+        return err == cudaSuccess ? RFX_OK : cuda_fail(err, "channelize, 1024 channels");
     }
     cudaError_t err = rfx::chan_branch_launch(x, taps, z, frames, plan->channels, num_taps,
                                               stream, format);
