@@ -1224,18 +1224,70 @@ cudaError_t fir_batch_tc_launch(const rfx_fir_capture* captures, int count, cuda
 
 namespace {
 
-// Cost of a work unit in microseconds of one SM, for the partition. Measured on GB300 with this
-// kernel (batch plans of each tap count of the 256-capture workload alone, CUDA-graph replay):
-// a long-filter tile of 96 blocks takes 16.4 SM-us at 511 taps (C = 4) and 18.7 at 1025
-// (C = 8); a plain tile of 2304 outputs 1.66, 2.27, 3.90, 6.54, 12.6 and 24.7 SM-us at 31, 63,
-// 127, 255, 511 and 1025 taps.
-double tc_tile_us(int C) { return 13.5 + 0.58 * static_cast<double>(C + 1); }
-double plain_tile_us(int num_taps) { return 1.0 + 0.0233 * static_cast<double>(num_taps); }
-// A resident-window tile of 48 blocks (batch plans as above: 3.0, 2.9 and 3.6 SM-us at 31, 63
-// and 127 taps, 4.2 at 255; C = 3 scaled from single captures of 2^24 samples, 2.98, 3.82 and
-// 4.69 SM-us for C = 1, 2, 3), and the tap strip built per capture.
-double win_tile_us(int C) { return C == 1 ? 3.1 : C == 2 ? 4.2 : 5.2; }
-constexpr double kWinStripUs = 1.0;
+// Costs for the partition, in microseconds of one SM: a tile, what a block pays to start on a capture
+// (its tap strip, the pipeline emptied before it, its first tile's scale), and to start a phase. Fitted
+// to the times of 1231 blocks' phases in eight batches of 64 to 256 captures of 2^12 to 2^17 .. 2^22
+// samples, each of 31 to 1025 taps (rms error 3 to 7 %): a long-filter tile of 96 blocks 15.2 at 511
+// taps (C = 4) and 16.6 at 1025 (C = 8), 6.9 per capture, 3.3 per phase; a window tile of 48 blocks
+// 2.39, 2.46 and 2.65 at 31, 63 and 127 taps (C = 1), 3.39 at 255 (C = 2), 1.9 and 3.2 per capture,
+// 4.2 and 4.6 per phase; C = 3 scaled from single captures (2.98, 3.82, 4.69 for C = 1, 2, 3). Plain
+// tiles of 2304 outputs (batch plans of one tap count): 1.66, 2.27, 3.90, 6.54, 12.6 and 24.7 at 31,
+// 63, 127, 255, 511 and 1025 taps.
+struct Cost {
+    double tile;
+    double start;
+};
+Cost tc_cost(int C) { return {13.9 + 0.34 * static_cast<double>(C), 6.9}; }
+Cost win_cost(int C, int num_taps)
+{
+    return C == 1   ? Cost{2.3 + 0.0027 * static_cast<double>(num_taps), 1.9}
+           : C == 2 ? Cost{3.4, 3.2}
+                    : Cost{4.2, 3.2};
+}
+Cost plain_cost(int num_taps) { return {1.0 + 0.0233 * static_cast<double>(num_taps), 0.0}; }
+// Phases in the order a block runs them: long-filter items, window items of C = 1, 2, 3, plain tiles.
+constexpr int kPhases = tcw::kCMax + 2;
+constexpr double kPhaseUs[kPhases] = {3.3, 4.2, 4.6, 4.6, 2.0};
+
+// A capture's tiles on the work line.
+struct Run {
+    int phase;
+    int tiles;
+    Cost cost;
+};
+
+// Cuts the line into contiguous pieces, each as long as it can be within `limit` (at least a tile);
+// ends[b]: units in the pieces up to b, counted over the whole line. Returns false if there are more
+// than `pieces`.
+bool cut_line(const std::vector<Run>& line, double limit, int pieces, std::vector<int>* ends)
+{
+    ends->clear();
+    double used = 0.0;
+    int phase = -1;
+    int unit = 0;
+    for (const Run& run : line) {
+        for (int left = run.tiles; left > 0;) {
+            const double start = run.cost.start + (run.phase != phase ? kPhaseUs[run.phase] : 0.0);
+            const double room = (limit - used - start) / run.cost.tile;
+            if (room < 1.0 && used > 0.0) {
+                ends->push_back(unit);
+                if (static_cast<int>(ends->size()) >= pieces) {
+                    return false;
+                }
+                used = 0.0;
+                phase = -1;
+                continue;
+            }
+            const int n = room < 1.0 ? 1 : room < left ? static_cast<int>(room) : left;
+            used += start + n * run.cost.tile;
+            phase = run.phase;
+            unit += n;
+            left -= n;
+        }
+    }
+    ends->push_back(unit);
+    return true;
+}
 
 constexpr int kPlainGroupsMax = kThreads / kPlainThreads;   // 3
 constexpr uint32_t kSmemMax = 227u * 1024u;
@@ -1290,13 +1342,11 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
     // Resident-window captures by blocks reached back (C = 1, 2, 3), their maps and costs.
     std::vector<tcw::WinCapture> wc[tcw::kCMax];
     std::vector<CUtensorMap> wm[tcw::kCMax];
-    std::vector<double> wcost[tcw::kCMax];
-    std::vector<double> cost;       // per work unit: tensor-core items, then plain tiles
+    std::vector<Run> runs[kPhases];   // the work line, phase by phase
     int kmax_plain = 0;
     int cmax = 0;
     int items = 0;
     int ptiles = 0;
-    std::vector<double> plain_cost;
     for (int i = 0; i < count; ++i) {
         const rfx_fir_capture& c = captures[i];
         if (c.num_samples == 0) {
@@ -1325,9 +1375,7 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
             wm[C - 1].push_back(m);
             const int tiles = static_cast<int>(((c.num_samples + kB - 1) / kB + tcw::kNB - 1) /
                                                tcw::kNB);
-            for (int t = 0; t < tiles; ++t) {
-                wcost[C - 1].push_back(win_tile_us(C) + (t == 0 ? kWinStripUs : 0.0));
-            }
+            runs[C].push_back(Run{C, tiles, win_cost(C, c.num_taps)});
         } else if (use_tc) {
             BatchCap b{};
             b.x = static_cast<const float2*>(c.x);
@@ -1351,9 +1399,7 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
             if (err != cudaSuccess) {
                 return err;
             }
-            for (int t = 0; t < b.tiles; ++t) {
-                cost.push_back(tc_tile_us(b.C));
-            }
+            runs[0].push_back(Run{0, b.tiles, tc_cost(b.C)});
             tc.push_back(b);
             xmaps.push_back(xm);
             smaps.push_back(sm);
@@ -1368,26 +1414,26 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
             const int tiles =
                 static_cast<int>((c.num_samples + kPlainTileOutputs - 1) / kPlainTileOutputs);
             ptiles += tiles;
-            for (int t = 0; t < tiles; ++t) {
-                plain_cost.push_back(plain_tile_us(c.num_taps));
-            }
+            runs[kPhases - 1].push_back(Run{kPhases - 1, tiles, plain_cost(c.num_taps)});
             kmax_plain = std::max(kmax_plain, c.num_taps);
             pl.push_back(q);
         }
     }
-    // The unit line: tensor-core items, window items (C = 1, 2, 3), plain tiles.
-    int wbase[tcw::kCMax];
-    int wunits[tcw::kCMax];
+    // The work line: the phases' captures one after another; first unit and units of each phase.
+    std::vector<Run> line;
+    int base[kPhases + 1] = {};
     int nwin = 0;
-    for (int ci = 0; ci < tcw::kCMax; ++ci) {
-        wbase[ci] = static_cast<int>(cost.size());
-        wunits[ci] = static_cast<int>(wcost[ci].size());
-        cost.insert(cost.end(), wcost[ci].begin(), wcost[ci].end());
-        nwin += static_cast<int>(wc[ci].size());
+    for (int ph = 0; ph < kPhases; ++ph) {
+        line.insert(line.end(), runs[ph].begin(), runs[ph].end());
+        base[ph + 1] = base[ph];
+        for (const Run& run : runs[ph]) {
+            base[ph + 1] += run.tiles;
+        }
     }
-    const int pbase = static_cast<int>(cost.size());
-    cost.insert(cost.end(), plain_cost.begin(), plain_cost.end());
-    const int units = static_cast<int>(cost.size());
+    for (const auto& list : wc) {
+        nwin += static_cast<int>(list.size());
+    }
+    const int units = base[kPhases];
     auto* plan = new BatchPlan{};
     plan->tc_caps = static_cast<int>(tc.size()) + nwin;
     plan->plain_caps = static_cast<int>(pl.size());
@@ -1451,37 +1497,43 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
         return cudaErrorInvalidValue;
     }
 
-    // Partition: the units on one line (tensor-core items, then plain tiles), cut into grid
-    // contiguous pieces of about equal cost; blocks of the first pieces run tensor-core items
-    // while the last ones run plain tiles, so tensor-bound and memory-bound work overlap.
-    const int grid = std::min({sms, kBatchCtas, units});
-    std::vector<double> prefix(units + 1, 0.0);
-    for (int u = 0; u < units; ++u) {
-        prefix[u + 1] = prefix[u] + cost[u];
+    // Partition: the line cut into at most one contiguous piece per SM, the longest piece as short as
+    // the costs allow (bisected); blocks of the first pieces run long-filter items while the last
+    // ones run windows and plain tiles, so tensor-bound and memory-bound work overlap. Measured with
+    // the costs above against equal shares of tile costs alone (busiest block / mean of all, us): 256
+    // captures of up to 2^22 samples 907 / 794 -> 865 / 797, 200 of up to 2^18 124 / 95 -> 110 / 96,
+    // 100 of up to 2^17 49 / 29 -> 39 / 29; back to back 896 -> 863, 129 -> 113 and 60 -> 49.
+    int grid = std::min({sms, kBatchCtas, units});
+    std::vector<int> ends;
+    double low = 0.0;
+    double high = 0.0;
+    for (const Run& run : line) {
+        high += run.tiles * run.cost.tile + run.cost.start + kPhaseUs[run.phase];
     }
+    for (int step = 0; step < 40; ++step) {
+        const double mid = 0.5 * (low + high);
+        (cut_line(line, mid, grid, &ends) ? high : low) = mid;
+    }
+    if (!cut_line(line, high, grid, &ends)) {
+        delete plan;
+        return cudaErrorInvalidValue;   // not reached: the whole line fits one piece
+    }
+    grid = static_cast<int>(ends.size());
     std::vector<int> cta_item(grid + 1), cta_plain(grid + 1);
     std::vector<int> cta_win[tcw::kCMax];
     for (auto& cw : cta_win) {
         cw.assign(grid + 1, 0);
     }
-    for (int b = 0; b <= grid; ++b) {
-        int u = b == grid ? units
-                          : static_cast<int>(std::lower_bound(prefix.begin(), prefix.end(),
-                                                              prefix[units] * b / grid) -
-                                             prefix.begin());
-        u = std::min(u, units);
-        cta_item[b] = std::min(u, items);
+    for (int b = 1; b <= grid; ++b) {
+        // Units of phase ph in the pieces before block b.
+        auto in_phase = [&](int ph) {
+            return std::min(std::max(ends[b - 1] - base[ph], 0), base[ph + 1] - base[ph]);
+        };
+        cta_item[b] = in_phase(0);
         for (int ci = 0; ci < tcw::kCMax; ++ci) {
-            cta_win[ci][b] = std::min(std::max(u - wbase[ci], 0), wunits[ci]);
+            cta_win[ci][b] = in_phase(ci + 1);
         }
-        cta_plain[b] = std::max(u - pbase, 0);
-    }
-    for (int b = 1; b <= grid; ++b) {   // monotone after rounding
-        cta_item[b] = std::max(cta_item[b], cta_item[b - 1]);
-        for (int ci = 0; ci < tcw::kCMax; ++ci) {
-            cta_win[ci][b] = std::max(cta_win[ci][b], cta_win[ci][b - 1]);
-        }
-        cta_plain[b] = std::max(cta_plain[b], cta_plain[b - 1]);
+        cta_plain[b] = in_phase(kPhases - 1);
     }
 
     // One device buffer: capture table, tensor maps (128-byte aligned), block ranges, plain
