@@ -106,6 +106,7 @@ struct Ctrl {
     int ex[kScales];                     // sample scale exponent of a tile
     int ehr[kScales];                    // tap scale exponent of a tile's capture
     uint32_t tap_max;
+    uint32_t first_max;                  // of the first tile's window (one tap set)
 };
 static_assert(sizeof(Ctrl) <= 1024, "control block");
 
@@ -261,7 +262,40 @@ __device__ __forceinline__ void build_strip(uint32_t hi, uint32_t lo, const floa
     }
 }
 
-// The pipeline over the block's tiles of `src`. `smem` is the dynamic shared memory (the layout
+// Initialises the control block (one thread, before a block barrier).
+template <int S>
+__device__ __forceinline__ void tcw_init(Ctrl& ctl)
+{
+    for (int i = 0; i < S; ++i) {
+        mbar_init(smem_u32(&ctl.full[i]), kProducerWarps);
+        mbar_init(smem_u32(&ctl.empty[i]), 1);
+    }
+    for (int i = 0; i < kWins; ++i) {
+        mbar_init(smem_u32(&ctl.win_full[i]), 1);
+        mbar_init(smem_u32(&ctl.win_empty[i]), kProducerWarps);
+    }
+    for (int i = 0; i < 2; ++i) {
+        mbar_init(smem_u32(&ctl.hfull[i]), 1);
+        mbar_init(smem_u32(&ctl.hempty[i]), kDrainWarps);
+        mbar_init(smem_u32(&ctl.xfull[i]), 1);
+        mbar_init(smem_u32(&ctl.xempty[i]), kDrainWarps);
+        mbar_init(smem_u32(&ctl.pready[i]), kScanWarps);
+        mbar_init(smem_u32(&ctl.strip_ready[i]), kScanWarps);
+        mbar_init(smem_u32(&ctl.strip_free[i]), 1);
+    }
+    for (int i = 0; i < kScales; ++i) {
+        mbar_init(smem_u32(&ctl.sready[i]), 1);
+    }
+    mbar_init(smem_u32(&ctl.patched), kScanWarps);
+    mbar_init(smem_u32(&ctl.teardown), 1);
+    ctl.abort = 0;
+    ctl.tap_max = 0;
+    ctl.first_max = 0;
+    fence_mbar_init();
+}
+
+// The pipeline over the block's tiles of `src`. With one tap set (not kMulti) the caller has run
+// tcw_init and synchronised the block. `smem` is the dynamic shared memory (the layout
 // from offset 1024), `ctl` its control block (anywhere outside the layout), `tmem` 512 columns
 // this block owns, `fault` the fault word. Every thread of the block calls it (kThreads of them:
 // warps beyond the roles return at the final barrier) and returns after a block barrier.
@@ -320,53 +354,99 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
     auto strip_slot = [](int occ) { return kStrips == 2 ? (occ & 1) : 0; };
     auto strip_use = [](int occ) { return kStrips == 2 ? (occ >> 1) : occ; };
 
-    // ---- setup: barriers, the first windows, the tap strip of a single capture -------------
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < stages; ++i) {
-            mbar_init(smem_u32(&ctl.full[i]), kProducerWarps);
-            mbar_init(smem_u32(&ctl.empty[i]), 1);
+    // The capture's last, partial block lies outside its tensor map (the copy read zeros): where the
+    // window at `win` of its tile t holds that row (only one tile of a capture does), `threads`
+    // threads store its samples there, ordered before the TMA that refills the window later. True
+    // if so (the same for all of them): they wait for each other before they read the window.
+    auto patch_tail = [&](const WinCapture& cap, long long t, uint32_t win, int tid, int threads) {
+        const long long full_blocks = cap.n / kB;
+        const int tail = static_cast<int>(cap.n - full_blocks * kB);
+        const long long rel = full_blocks - (t * NB - C);
+        if (tail == 0 || rel < 0 || rel >= rows) {
+            return false;
         }
-        for (int i = 0; i < wins; ++i) {
-            mbar_init(smem_u32(&ctl.win_full[i]), 1);
-            mbar_init(smem_u32(&ctl.win_empty[i]), kProducerWarps);
+        const uint32_t row = win + static_cast<uint32_t>(rel) * 256u * es;
+        for (int i = tid; i < tail; i += threads) {
+            const long long sidx = full_blocks * kB + i;
+            if constexpr (kFmt == 0) {
+                const float2 v = __ldg(static_cast<const float2*>(cap.x) + sidx);
+                sts64(row + static_cast<uint32_t>(i) * 8u, pack2(v.x, v.y));
+            } else if constexpr (kFmt == 1) {
+                sts32(row + static_cast<uint32_t>(i) * 4u,
+                      __ldg(static_cast<const unsigned int*>(cap.x) + sidx));
+            } else {
+                const unsigned short v = __ldg(static_cast<const unsigned short*>(cap.x) + sidx);
+                asm volatile("st.shared.u16 [%0], %1;"
+                             ::"r"(row + static_cast<uint32_t>(i) * 2u), "h"(v)
+                             : "memory");
+            }
         }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(smem_u32(&ctl.hfull[i]), 1);
-            mbar_init(smem_u32(&ctl.hempty[i]), kDrainWarps);
-            mbar_init(smem_u32(&ctl.xfull[i]), 1);
-            mbar_init(smem_u32(&ctl.xempty[i]), kDrainWarps);
-            mbar_init(smem_u32(&ctl.pready[i]), kScanWarps);
-            mbar_init(smem_u32(&ctl.strip_ready[i]), kScanWarps);
-            mbar_init(smem_u32(&ctl.strip_free[i]), 1);
+        fence_proxy_async_smem();
+        return true;
+    };
+    // Largest |component| of the window at `win`, over the pairs of `threads` threads' thread tid.
+    auto scan_window = [&](uint32_t win, int tid, int threads) {
+        uint32_t m = 0;
+#pragma unroll 4
+        for (int f = tid; f < rows * 64; f += threads) {
+            m = max(m, absmax4(lds_pair(win + static_cast<uint32_t>(f) * kPairBytes, kFmt)));
         }
-        for (int i = 0; i < kScales; ++i) {
-            mbar_init(smem_u32(&ctl.sready[i]), 1);
-        }
-        mbar_init(smem_u32(&ctl.patched), kScanWarps);
-        mbar_init(smem_u32(&ctl.teardown), 1);
-        ctl.abort = 0;
-        ctl.tap_max = 0;
-        fence_mbar_init();
-        for (int k = 0; k < wins && k < my_tiles; ++k) {
-            issue_window(k);   // thread 0 is the copy warp's issuing lane
-        }
-    }
+        return __reduce_max_sync(0xFFFFFFFFu, m);
+    };
+
+    // ---- setup: the first windows, the tap strip and the first tile's scale ------------------
     int eh_single = 0;         // the tap scale of a single capture
-    if constexpr (!kMulti) {
+    if constexpr (kMulti) {
+        if (threadIdx.x == 0) {
+            tcw_init<S>(ctl);
+            for (int k = 0; k < wins && k < my_tiles; ++k) {
+                issue_window(k);   // thread 0 is the copy warp's issuing lane
+            }
+        }
+    } else {
+        // One tap set (the caller has initialised the barriers and synchronised the block, while the
+        // kernel before it in the stream was still running). The
+        // second and third window are asked for once the taps have arrived: behind three windows
+        // of every SM they came a microsecond later. The first tile's scale is taken by all
+        // threads: two scan warps took 0.4 to 0.9 us for it, with nothing else to do meanwhile.
+        // Measured with the three together (63 taps, us): 2^16 samples 5.05 -> 4.61, 2^20 8.52 ->
+        // 8.04, 2^24 52.5 -> 51.1; 1025 taps, 2^16 samples 10.99 -> 10.28.
+        if (threadIdx.x == 0 && my_tiles > 0) {
+            issue_window(0);
+        }
         const WinCapture& cap = src.capture(0);
         uint32_t m = 0;
         for (int k = threadIdx.x; k < cap.num_taps; k += kThreads) {
             m = max(m, absbits(__ldg(cap.taps + k)));
         }
         m = __reduce_max_sync(0xFFFFFFFFu, m);
-        __syncthreads();   // tap_max initialised
         if (lane == 0 && m != 0) {
             atomicMax(&ctl.tap_max, m);
         }
         __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < wins && k < my_tiles; ++k) {
+                issue_window(k);
+            }
+        }
         eh_single = scale_exponent(ctl.tap_max);
         build_strip<C>(strip_hi(0), strip_lo(0), cap.taps, cap.num_taps, eh_single,
                        threadIdx.x, kThreads);
+        if (my_tiles > 0) {
+            TcwCursor cur;
+            long long t;
+            src.locate(0, cur, t);
+            const uint32_t win = sbase + lay.win0;
+            // (A give-up shows in *abort, which every role tests before its first tile.)
+            if (mbar_wait_bounded(smem_u32(&ctl.win_full[0]), 0, fault, kFaultTileLoad, abort)) {
+                patch_tail(src.capture(cur.idx), t, win, threadIdx.x, kThreads);
+            }
+            __syncthreads();
+            const uint32_t w = scan_window(win, threadIdx.x, kThreads);
+            if (lane == 0 && w != 0) {
+                atomicMax(&ctl.first_max, w);
+            }
+        }
     }
     fence_proxy_async_smem();
     fence_before();
@@ -756,7 +836,16 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
         int cap_now = -1;
         int patches = 0;   // partial blocks written (phases of `patched`)
         int eh = eh_single;
-        for (int j = 0; j < my_tiles && !*abort; ++j) {
+        constexpr int kScanned = kMulti ? 0 : 1;   // tiles whose scale the setup took
+        if constexpr (!kMulti) {
+            if (stid == 0 && my_tiles > 0) {
+                ctl.ex[0] = min(scale_exponent(ctl.first_max), 127);
+                ctl.ehr[0] = eh;
+                mbar_arrive(smem_u32(&ctl.sready[0]));
+            }
+        }
+        for (int j = kScanned; j < my_tiles && !*abort; ++j) {
+            const int s = j - kScanned;
             long long t;
             src.locate(j, cur, t);
             const WinCapture& cap = src.capture(cur.idx);
@@ -780,33 +869,9 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
                 break;
             }
             const uint32_t win = sbase + lay.win0 + static_cast<uint32_t>(wb) * lay.win;
-            // The capture's last, partial block lies outside its tensor map (the copy read
-            // zeros): its stored samples go into their window row (only one tile of a capture
-            // holds that row), then the scan warps wait for each other. With a list of
-            // captures this happens once per capture: the barrier's phase counts them.
-            const long long full_blocks = cap.n / kB;
-            const int tail = static_cast<int>(cap.n - full_blocks * kB);
-            const long long rel = full_blocks - (t * NB - C);
-            if (tail > 0 && rel >= 0 && rel < rows) {   // uniform across the scan warps
-                const uint32_t row = win + static_cast<uint32_t>(rel) * 256u * es;
-                for (int i = stid; i < tail; i += kScanWarps * 32) {
-                    const long long sidx = full_blocks * kB + i;
-                    if constexpr (kFmt == 0) {
-                        const float2 v = __ldg(static_cast<const float2*>(cap.x) + sidx);
-                        sts64(row + static_cast<uint32_t>(i) * 8u, pack2(v.x, v.y));
-                    } else if constexpr (kFmt == 1) {
-                        sts32(row + static_cast<uint32_t>(i) * 4u,
-                              __ldg(static_cast<const unsigned int*>(cap.x) + sidx));
-                    } else {
-                        const unsigned short v =
-                            __ldg(static_cast<const unsigned short*>(cap.x) + sidx);
-                        asm volatile("st.shared.u16 [%0], %1;"
-                                     ::"r"(row + static_cast<uint32_t>(i) * 2u), "h"(v)
-                                     : "memory");
-                    }
-                }
-                // The window is refilled by TMA later: order these writes before that.
-                fence_proxy_async_smem();
+            // The capture's partial last block, then the scan warps wait for each other. With a list
+            // of captures this happens once per capture: the barrier's phase counts them.
+            if (patch_tail(cap, t, win, stid, kScanWarps * 32)) {
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(smem_u32(&ctl.patched));
@@ -817,27 +882,21 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
                 }
                 ++patches;
             }
-            uint32_t m = 0;
-            constexpr int pairs = rows * 64;
-#pragma unroll 4
-            for (int f = stid; f < pairs; f += kScanWarps * 32) {
-                m = max(m, absmax4(lds_pair(win + static_cast<uint32_t>(f) * kPairBytes, kFmt)));
-            }
-            m = __reduce_max_sync(0xFFFFFFFFu, m);
-            // (Two maximum buffers suffice: a warp writes tile j + 2's only after every warp has
-            // arrived for tile j + 1, i.e. after it read tile j's.)
+            const uint32_t m = scan_window(win, stid, kScanWarps * 32);
+            // (Two maximum buffers suffice: a warp writes scan s + 2's only after every warp has
+            // arrived for scan s + 1, i.e. after it read scan s's.)
             if (lane == 0) {
-                ctl.pmax[j & 1][sw] = m;
-                mbar_arrive(smem_u32(&ctl.pready[j & 1]));
+                ctl.pmax[s & 1][sw] = m;
+                mbar_arrive(smem_u32(&ctl.pready[s & 1]));
             }
-            if (!mbar_wait_bounded(smem_u32(&ctl.pready[j & 1]), (j >> 1) & 1, fault,
+            if (!mbar_wait_bounded(smem_u32(&ctl.pready[s & 1]), (s >> 1) & 1, fault,
                                    kFaultScale, abort)) {
                 break;
             }
             uint32_t tmax = 0;
 #pragma unroll
             for (int w = 0; w < kScanWarps; ++w) {
-                tmax = max(tmax, *reinterpret_cast<volatile uint32_t*>(&ctl.pmax[j & 1][w]));
+                tmax = max(tmax, *reinterpret_cast<volatile uint32_t*>(&ctl.pmax[s & 1][w]));
             }
             if (stid == 0) {
                 ctl.ex[j % kScales] = min(scale_exponent(tmax), 127);

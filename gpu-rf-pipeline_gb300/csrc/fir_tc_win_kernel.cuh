@@ -32,6 +32,9 @@ fir_tcw_kernel(const __grid_constant__ CUtensorMap wmap, const void* __restrict_
     if (warp == tcw::kMmaWarp) {
         tc::tmem_alloc(smem_u32(tmem_slot), tcw::kTmemCols);
     }
+    if (threadIdx.x == 0) {
+        tcw::tcw_init<8>(ctl);
+    }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
