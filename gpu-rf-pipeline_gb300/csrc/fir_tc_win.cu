@@ -13,10 +13,16 @@
 // each window row, N index 2 j + {0: I, 1: Q}). Chunk C of a K-step whose taps are all zero
 // (16 st <= C B - K - 15) is skipped: 63 taps need 12 of the 16 chunk-steps.
 //
-// What differs from fir_tc.cu (which keeps the longer filters: at N = 96 the MMAs read 7 KB of
-// operands per 48 tensor cycles, more than shared memory delivers, so from about 500 taps on
-// fir_tc.cu's N = 192 tiles are faster: measured 123 against 120 us at 511 taps, 162 against
-// 141 us at 1025):
+// What differs from fir_tc.cu (which keeps the longest filters: its N = 192 tiles spread a tap
+// matrix's read over twice the columns):
+//  * tap matrices (128 x 16 FP16) sit in tensor memory beside the accumulators as far as its columns
+//    go: both splits' up to C = 1 and the high split's up to C = 3 at 32 blocks, two chunks of the
+//    high split at 48. Read from the strip in shared memory, 4 KB per MMA, they set the MMAs' pace
+//    (99 cycles an MMA at N = 96 against 51 of the tensor cores) and took the bandwidth that the
+//    copies, the scan and the converters need. 2^24 samples (us): 63 taps 51.1 -> 46.1, 255 taps 70.4
+//    -> 60.5, 385 taps 82.6 -> 73; 2^20 samples, 255 taps 10.8 -> 10.1, 1025 taps 19.2 -> 18.2. Tiles of
+//    8 and 16 blocks at C <= 2 keep the strip: one such tile is over before the copies to tensor
+//    memory are paid back (63 taps, 2^16 samples 4.6 against 5.0);
 //  * the whole window arrives by ONE 2-D TMA copy (rows of 1 KB for cf32) into a ring of three
 //    window buffers, issued by a copy warp as soon as a buffer is converted: each sample
 //    crosses HBM once and the TMA engine once (fir_tc.cu copies it twice: a scan slice and a
@@ -85,12 +91,13 @@ bool fir_tcw_supported(int num_taps)
 // C = blocks reached back to). Resident window: a first tile through the whole pipeline, then one
 // step per further tile; long-filter form (96 blocks a tile): one step per tile. So short captures
 // take small tiles on more SMs, middling ones the tile that fills the last round, long ones the
-// largest tile of the window form or, beyond 385 taps, the long-filter form. Measured, 63 / 255 /
-// 385 taps: one tile of 8, 16, 24, 32, 48 blocks 4.9 / 6.3 / 7.1, 5.1 / 6.5 / 7.4, 5.8 / 7.0 / 7.9,
-// 6.0 / 7.4 / 8.3, 6.8 / 8.5 / 9.4, each further one 1.6 / 2.4 / 3.1 (8 blocks) to 2.6 / 3.5 / 4.4
-// (48); 511 / 1025 taps: 2^16 samples 7.9 / 11.0 (16 blocks) against 19.0 / 23.6 in the long-filter
-// form, 2^20 13.7 / 20.0 (32) against 20.2 / 25.0, 2^22 36.4 / 56.5 against 50.3 / 58.8, 2^23
-// 65.2 / 105.1 against 73.0 / 85.2.
+// largest tile of the window form or, beyond 385 taps, the long-filter form where it is faster.
+// Measured, 63 / 255 / 385 taps: one tile of 8, 16, 24, 32, 48 blocks 4.6 / 5.9 / 6.8, 5.0 / 6.2 / 7.1,
+// 5.6 / 6.6 / 7.4, 5.8 / 7.0 / 7.3, 6.0 / 7.3 / 8.3, each further one 1.5 / 2.4 / 1.9 (8 blocks) to
+// 2.3 / 3.0 / 3.8 (48); 511 / 1025 taps: 2^16 samples 7.6 / 10.5 (16 blocks) against 18.9 / 24.3 in the
+// long-filter form, 2^20 12.5 / 18.3 (32) against 20.5 / 25.3, 2^22 31.9 / 51.2 against 50.6 / 58.6,
+// 2^23 56.0 / 94.8 against 72.6 / 83.9, 2^24 101 / 175 against 118 / 138 (768 taps 143 against 125).
+// The rule's choice was within 0.2 % of the best on average over 144 cases, 7 % at worst.
 int fir_tcw_tile_blocks(int num_taps, long long n)
 {
     int device = 0;
@@ -117,8 +124,10 @@ int fir_tcw_tile_blocks(int num_taps, long long n)
         if (!fir_tcw_takes(num_taps, nb)) {
             continue;
         }
-        const double us = 4.0 + 0.75 * C + (0.045 + 0.004 * C) * nb +
-                          (rounds(nb) - 1.0) * (0.75 + 0.53 * C + (0.02 + 0.007 * C) * nb);
+        const double step = C <= tcw::kCMax ? 0.75 + 0.53 * C + (0.02 + 0.007 * C) * nb
+                                            : 0.2 + 0.5 * C + (0.02 + 0.006 * C) * nb;
+        const double us =
+            4.0 + 0.75 * C + (0.045 + 0.004 * C) * nb + (rounds(nb) - 1.0) * step;
         if (us < best_us) {
             best_us = us;
             best = nb;

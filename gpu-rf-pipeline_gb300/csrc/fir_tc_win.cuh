@@ -27,7 +27,6 @@ using namespace tc;
 
 constexpr int kB = 128;                   // outputs per block = MMA M
 constexpr int kNB = 48;                   // blocks per tile, at most; MMA N = 2 * blocks
-constexpr int kN = 2 * kNB;               // columns of an accumulator
 constexpr int kCMax = 3;                  // blocks a block reaches back to, at most (385 taps)
 constexpr int kSteps = kB / 16;           // K-steps of 16 samples per tile
 constexpr int kWins = 3;                  // window buffers
@@ -43,8 +42,7 @@ constexpr int kDrainWarps = 8;
 constexpr int kFirstScanWarp = kFirstDrainWarp + kDrainWarps;
 constexpr int kScanWarps = 2;
 constexpr int kThreads = (kFirstScanWarp + kScanWarps) * 32;
-constexpr uint32_t kTmemCols = 512;       // H0, H1, X0, X1 of kN columns each: 384 used
-constexpr uint32_t kXCol = 2 * kN;        // first column of X0
+constexpr uint32_t kTmemCols = 512;       // H0, H1, X0, X1 of 2 NB columns each, then taps
 constexpr uint32_t kSmemMax = 227u * 1024u;
 
 // One capture as the pipeline sees it.
@@ -311,7 +309,20 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
     constexpr uint32_t kPairBytes = 4u * es;   // two samples as stored
     constexpr int rows = NB + C;
     constexpr uint32_t kIdesc = idesc_f16(kB, 2 * NB);
-    static_assert(NB % 8 == 0 && NB <= kNB, "MMA N = 2 NB is a multiple of 16, at most kN");
+    constexpr uint32_t kN = 2 * NB;           // columns of an accumulator
+    constexpr uint32_t kXCol = 2 * kN;        // first column of X0
+    // Tap matrices in tensor memory (one tap set; fir_tc_win.cu gives the reason): chunk c's eight
+    // K-steps take 64 columns per split, the high split's chunks first, then the low split's, as
+    // far as the columns go. The other MMAs read the strip in shared memory.
+    constexpr int kChunkCols = 8 * kSteps;
+    constexpr int kRoom = kMulti || (NB <= 16 && C <= 2)
+                              ? 0
+                              : static_cast<int>(kTmemCols - 4 * kN) / kChunkCols;
+    constexpr int kHiChunks = kRoom < C + 1 ? kRoom : C + 1;
+    constexpr int kLoChunks = kRoom - kHiChunks < C + 1 ? kRoom - kHiChunks : C + 1;
+    constexpr uint32_t kHiCol = 4 * kN;
+    constexpr uint32_t kLoCol = kHiCol + kHiChunks * kChunkCols;
+    static_assert(NB % 8 == 0 && NB <= kNB, "MMA N = 2 NB is a multiple of 16");
     constexpr int hks = kSteps < kHGroup / (C + 1) ? kSteps : kHGroup / (C + 1);
     constexpr int groups = (kSteps + hks - 1) / hks;
     constexpr int wins = kWins;
@@ -475,6 +486,10 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
         const uint32_t stage_units = lay.stage >> 4;
         const uint32_t split_units = lay.split >> 4;
         bool stop = false;
+        if constexpr (kRoom > 0) {
+            asm volatile("bar.sync 1, %0;" ::"n"((kDrainWarps + 1) * 32) : "memory");
+            fence_after();   // the drain warps' tap matrices
+        }
         int u = 0;     // K-steps issued (block-wide numbering)
         int g = 0;     // H groups issued
         TcwCursor cur;
@@ -538,18 +553,40 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
                     const uint32_t h_first = st == st0 ? 0u : 1u;
                     const uint32_t x_first = st == 0 ? 0u : 1u;
                     const int c_end = st >= st_cmax ? C + 1 : C;
+                    const uint32_t ta = tmem + static_cast<uint32_t>(8 * st);
                     if (elect_one()) {
-                        mma_f16<kIdesc>(h_acc, dah, dbh, h_first);
-                        mma_f16<kIdesc>(x_acc, dah, dbl, x_first);
-                        mma_f16_acc<kIdesc>(x_acc, dal, dbh);
-                        for (int c = 1; c < c_end; ++c) {
-                            dah -= 128;
-                            dal -= 128;
-                            dbh -= 2;
-                            dbl -= 2;
-                            mma_f16_acc<kIdesc>(h_acc, dah, dbh);
-                            mma_f16_acc<kIdesc>(x_acc, dah, dbl);
-                            mma_f16_acc<kIdesc>(x_acc, dal, dbh);
+#pragma unroll
+                        for (int c = 0; c <= C; ++c) {
+                            if (c < c_end) {
+                                if constexpr (kHiChunks > 0) {
+                                    if (c < kHiChunks) {
+                                        const uint32_t th = ta + kHiCol + c * kChunkCols;
+                                        if (c == 0) {
+                                            mma_f16_ta<kIdesc>(h_acc, th, dbh, h_first);
+                                            mma_f16_ta<kIdesc>(x_acc, th, dbl, x_first);
+                                        } else {
+                                            mma_f16_ta_acc<kIdesc>(h_acc, th, dbh);
+                                            mma_f16_ta_acc<kIdesc>(x_acc, th, dbl);
+                                        }
+                                    } else {
+                                        mma_f16_acc<kIdesc>(h_acc, dah, dbh);
+                                        mma_f16_acc<kIdesc>(x_acc, dah, dbl);
+                                    }
+                                } else {
+                                    mma_f16<kIdesc>(h_acc, dah, dbh, c == 0 ? h_first : 1u);
+                                    mma_f16<kIdesc>(x_acc, dah, dbl, c == 0 ? x_first : 1u);
+                                }
+                                if (c < kLoChunks) {
+                                    mma_f16_ta_acc<kIdesc>(
+                                        x_acc, ta + kLoCol + c * kChunkCols, dbh);
+                                } else {
+                                    mma_f16_acc<kIdesc>(x_acc, dal, dbh);
+                                }
+                                dah -= 128;
+                                dal -= 128;
+                                dbh -= 2;
+                                dbl -= 2;
+                            }
                         }
                         mma_commit(smem_u32(&ctl.empty[slot]));
                     }
@@ -678,6 +715,33 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
         const int r = kB - 1 - (quarter * 32 + lane);          // output row of this TMEM lane
         const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) +
                                    static_cast<uint32_t>(half * NB);
+        if constexpr (kRoom > 0) {
+            // The tap matrices, while the first tile is converted. Matrix (c, st), row m (lane m):
+            // strip elements 16 C + 2 st - 16 c + m / 8 and the next, row m % 8 of each.
+            const int m = quarter * 32 + lane;
+            const uint32_t row_off = static_cast<uint32_t>(16 * C + m / 8) * 128u +
+                                     static_cast<uint32_t>(m % 8) * 16u;
+            const uint32_t dst = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kHiCol;
+            constexpr int kMatrices = (kHiChunks + kLoChunks) * kSteps;
+#pragma unroll 4
+            for (int i = half; i < kMatrices; i += kDrainWarps / 4) {
+                const bool hi = i < kHiChunks * kSteps;
+                const int j = hi ? i : i - kHiChunks * kSteps;   // 8 c + st
+                const uint32_t from = (hi ? strip_hi(0) : strip_lo(0)) + row_off +
+                                      static_cast<uint32_t>(2 * (j % kSteps)) * 128u -
+                                      static_cast<uint32_t>(16 * (j / kSteps)) * 128u;
+                const float4 e0 = lds128(from);
+                const float4 e1 = lds128(from + 128u);
+                const uint32_t v[8] = {__float_as_uint(e0.x), __float_as_uint(e0.y),
+                                       __float_as_uint(e0.z), __float_as_uint(e0.w),
+                                       __float_as_uint(e1.x), __float_as_uint(e1.y),
+                                       __float_as_uint(e1.z), __float_as_uint(e1.w)};
+                tmem_st8(dst + static_cast<uint32_t>(8 * i), v);
+            }
+            tmem_wait_st();
+            fence_before();
+            asm volatile("bar.arrive 1, %0;" ::"n"((kDrainWarps + 1) * 32) : "memory");
+        }
         float acc[groups > 1 ? NB : 1];
 #pragma unroll
         for (int i = 0; i < (groups > 1 ? NB : 1); ++i) {

@@ -50,6 +50,30 @@ __device__ __forceinline__ void mma_f16_acc(uint32_t d_tmem, unsigned long long 
         : "memory");
 }
 
+// The same with A in tensor memory: row m in lane m, 16 FP16 of K in eight columns from a_tmem on,
+// two per column.
+template <uint32_t kIdesc>
+__device__ __forceinline__ void mma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, unsigned long long b,
+                                           uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b), "r"(kIdesc), "r"(accumulate)
+        : "memory");
+}
+
+template <uint32_t kIdesc>
+__device__ __forceinline__ void mma_f16_ta_acc(uint32_t d_tmem, uint32_t a_tmem,
+                                               unsigned long long b)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 1, 1;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b), "r"(kIdesc)
+        : "memory");
+}
+
 // One lane of a fully active warp (the same lane every time): the lane that issues a warp's
 // MMAs and commits. Running the issue loop on the whole warp and electing the issuer keeps
 // the loop's values (descriptors, TMEM addresses, counters) warp-uniform, so they can live in
@@ -111,6 +135,20 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&t)[8])
                  : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]),
                    "=r"(t[6]), "=r"(t[7])
                  : "r"(taddr));
+}
+
+// This warp's 32 lanes of eight columns from taddr on.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&t)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(taddr), "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]),
+                 "r"(t[6]), "r"(t[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_wait_st()
+{
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // 16 lanes x 256 bits, four times along the columns: for 8-column group j (registers 4j .. 4j+3)
