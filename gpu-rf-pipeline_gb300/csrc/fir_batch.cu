@@ -28,7 +28,8 @@
 // resident-window pipeline of fir_tc_win.cuh over its captures of 2 to 385 taps: one phase per
 // reach-back C = 1, 2, 3 (the window geometry is compile-time), each block taking a contiguous
 // range of that phase's 48-block tiles; the scan warps rebuild the tap strip at every capture
-// switch into one of two slots, the MMA warp freeing a slot after its capture's last tile. Last
+// switch into one of two slots, the MMA warp freeing a slot after its capture's last tile, and the
+// drain warps replace the tap matrices in tensor memory. Last
 // come the plain tiles of the captures below 2 taps (the plain kernel's tile function:
 // bit-exact). Tensor memory is allocated once per block for every phase.
 #include "fir_tc.cuh"
@@ -1227,65 +1228,66 @@ namespace {
 // Costs for the partition, in microseconds of one SM: a tile, what a block pays to start on a capture
 // (its tap strip, the pipeline emptied before it, its first tile's scale), and to start a phase. Fitted
 // to the times of 1231 blocks' phases in eight batches of 64 to 256 captures of 2^12 to 2^17 .. 2^22
-// samples, each of 31 to 1025 taps (rms error 3 to 7 %): a long-filter tile of 96 blocks 15.2 at 511
-// taps (C = 4) and 16.6 at 1025 (C = 8), 6.9 per capture, 3.3 per phase; a window tile of 48 blocks
-// 2.39, 2.46 and 2.65 at 31, 63 and 127 taps (C = 1), 3.39 at 255 (C = 2), 1.9 and 3.2 per capture,
-// 4.2 and 4.6 per phase; C = 3 scaled from single captures (2.98, 3.82, 4.69 for C = 1, 2, 3). Plain
+// samples, each of 31 to 1025 taps (rms error 3 to 8 %): a long-filter tile of 96 blocks 14.8 at 511
+// taps (C = 4) and 16.5 at 1025 (C = 8), 9.9 per capture; a window tile of 48 blocks 2.11, 2.16 and
+// 2.20 at 31, 63 and 127 taps (C = 1), 2.83 at 255 (C = 2), 2.5 and 4.1 per capture, 4.1 and 5.4 per
+// phase (2.39, 2.46, 2.65 and 3.39 a tile before their tap matrices were in tensor memory); C = 3
+// scaled from single captures. Plain
 // tiles of 2304 outputs (batch plans of one tap count): 1.66, 2.27, 3.90, 6.54, 12.6 and 24.7 at 31,
 // 63, 127, 255, 511 and 1025 taps.
 struct Cost {
     double tile;
     double start;
 };
-Cost tc_cost(int C) { return {13.9 + 0.34 * static_cast<double>(C), 6.9}; }
+Cost tc_cost(int C) { return {13.5 + 0.38 * static_cast<double>(C), 6.9}; }
 Cost win_cost(int C, int num_taps)
 {
-    return C == 1   ? Cost{2.3 + 0.0027 * static_cast<double>(num_taps), 1.9}
-           : C == 2 ? Cost{3.4, 3.2}
-                    : Cost{4.2, 3.2};
+    return C == 1   ? Cost{2.1 + 0.001 * static_cast<double>(num_taps), 2.5}
+           : C == 2 ? Cost{2.8, 4.1}
+                    : Cost{3.5, 4.1};
 }
 Cost plain_cost(int num_taps) { return {1.0 + 0.0233 * static_cast<double>(num_taps), 0.0}; }
 // Phases in the order a block runs them: long-filter items, window items of C = 1, 2, 3, plain tiles.
 constexpr int kPhases = tcw::kCMax + 2;
-constexpr double kPhaseUs[kPhases] = {3.3, 4.2, 4.6, 4.6, 2.0};
+constexpr double kPhaseUs[kPhases] = {3.3, 4.1, 5.4, 5.4, 2.0};
 
-// A capture's tiles on the work line.
+// A capture's tiles in its phase.
 struct Run {
-    int phase;
     int tiles;
     Cost cost;
 };
 
-// Cuts the line into contiguous pieces, each as long as it can be within `limit` (at least a tile);
-// ends[b]: units in the pieces up to b, counted over the whole line. Returns false if there are more
-// than `pieces`.
-bool cut_line(const std::vector<Run>& line, double limit, int pieces, std::vector<int>* ends)
+// Deals the phases' tiles, in order, to blocks 0, 1, ..., every block filled up to `longest` (from the
+// window phases on up to `rest`; at least a tile each): tiles[phase][block]. Returns false if they do
+// not fit `blocks` blocks.
+bool deal(const std::vector<Run> (&runs)[kPhases], double longest, double rest, int blocks,
+          std::vector<int> (&tiles)[kPhases])
 {
-    ends->clear();
-    double used = 0.0;
-    int phase = -1;
-    int unit = 0;
-    for (const Run& run : line) {
-        for (int left = run.tiles; left > 0;) {
-            const double start = run.cost.start + (run.phase != phase ? kPhaseUs[run.phase] : 0.0);
-            const double room = (limit - used - start) / run.cost.tile;
-            if (room < 1.0 && used > 0.0) {
-                ends->push_back(unit);
-                if (static_cast<int>(ends->size()) >= pieces) {
+    std::vector<double> used(blocks, 0.0);
+    int b = 0;
+    for (int ph = 0; ph < kPhases; ++ph) {
+        const double limit = ph == 0 ? longest : rest;
+        tiles[ph].assign(blocks, 0);
+        for (const Run& run : runs[ph]) {
+            for (int left = run.tiles; left > 0;) {
+                if (b == blocks) {
                     return false;
                 }
-                used = 0.0;
-                phase = -1;
-                continue;
+                const double start = run.cost.start + (tiles[ph][b] == 0 ? kPhaseUs[ph] : 0.0);
+                const double room = (limit - used[b] - start) / run.cost.tile;
+                const int n = room < 1.0 ? (used[b] == 0.0 ? 1 : 0)
+                              : room < left ? static_cast<int>(room)
+                                            : left;
+                if (n == 0) {
+                    ++b;
+                    continue;
+                }
+                used[b] += start + n * run.cost.tile;
+                tiles[ph][b] += n;
+                left -= n;
             }
-            const int n = room < 1.0 ? 1 : room < left ? static_cast<int>(room) : left;
-            used += start + n * run.cost.tile;
-            phase = run.phase;
-            unit += n;
-            left -= n;
         }
     }
-    ends->push_back(unit);
     return true;
 }
 
@@ -1342,7 +1344,7 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
     // Resident-window captures by blocks reached back (C = 1, 2, 3), their maps and costs.
     std::vector<tcw::WinCapture> wc[tcw::kCMax];
     std::vector<CUtensorMap> wm[tcw::kCMax];
-    std::vector<Run> runs[kPhases];   // the work line, phase by phase
+    std::vector<Run> runs[kPhases];
     int kmax_plain = 0;
     int cmax = 0;
     int items = 0;
@@ -1375,7 +1377,7 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
             wm[C - 1].push_back(m);
             const int tiles = static_cast<int>(((c.num_samples + kB - 1) / kB + tcw::kNB - 1) /
                                                tcw::kNB);
-            runs[C].push_back(Run{C, tiles, win_cost(C, c.num_taps)});
+            runs[C].push_back(Run{tiles, win_cost(C, c.num_taps)});
         } else if (use_tc) {
             BatchCap b{};
             b.x = static_cast<const float2*>(c.x);
@@ -1399,7 +1401,7 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
             if (err != cudaSuccess) {
                 return err;
             }
-            runs[0].push_back(Run{0, b.tiles, tc_cost(b.C)});
+            runs[0].push_back(Run{b.tiles, tc_cost(b.C)});
             tc.push_back(b);
             xmaps.push_back(xm);
             smaps.push_back(sm);
@@ -1414,26 +1416,23 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
             const int tiles =
                 static_cast<int>((c.num_samples + kPlainTileOutputs - 1) / kPlainTileOutputs);
             ptiles += tiles;
-            runs[kPhases - 1].push_back(Run{kPhases - 1, tiles, plain_cost(c.num_taps)});
+            runs[kPhases - 1].push_back(Run{tiles, plain_cost(c.num_taps)});
             kmax_plain = std::max(kmax_plain, c.num_taps);
             pl.push_back(q);
         }
     }
-    // The work line: the phases' captures one after another; first unit and units of each phase.
-    std::vector<Run> line;
-    int base[kPhases + 1] = {};
-    int nwin = 0;
+    int units = 0;
+    double all_us = 0.0;
     for (int ph = 0; ph < kPhases; ++ph) {
-        line.insert(line.end(), runs[ph].begin(), runs[ph].end());
-        base[ph + 1] = base[ph];
         for (const Run& run : runs[ph]) {
-            base[ph + 1] += run.tiles;
+            units += run.tiles;
+            all_us += run.tiles * run.cost.tile + run.cost.start + kPhaseUs[ph];
         }
     }
+    int nwin = 0;
     for (const auto& list : wc) {
         nwin += static_cast<int>(list.size());
     }
-    const int units = base[kPhases];
     auto* plan = new BatchPlan{};
     plan->tc_caps = static_cast<int>(tc.size()) + nwin;
     plan->plain_caps = static_cast<int>(pl.size());
@@ -1497,44 +1496,52 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
         return cudaErrorInvalidValue;
     }
 
-    // Partition: the line cut into at most one contiguous piece per SM, the longest piece as short as
-    // the costs allow (bisected); blocks of the first pieces run long-filter items while the last
-    // ones run windows and plain tiles, so tensor-bound and memory-bound work overlap. Measured with
-    // the costs above against equal shares of tile costs alone (busiest block / mean of all, us): 256
-    // captures of up to 2^22 samples 907 / 794 -> 865 / 797, 200 of up to 2^18 124 / 95 -> 110 / 96,
-    // 100 of up to 2^17 49 / 29 -> 39 / 29; back to back 896 -> 863, 129 -> 113 and 60 -> 49.
-    int grid = std::min({sms, kBatchCtas, units});
-    std::vector<int> ends;
+    // Partition: at most one block per SM, a contiguous range of each phase's tiles per block, the
+    // longest block as short as the costs allow (bisected), then the blocks that windows and plain
+    // tiles are left with as short as they can be: a batch of few tiles is as long as its one
+    // long-filter tile, and its windows need not queue for that time. Blocks of the first ranges run
+    // long-filter items while the last ones run windows and plain tiles, so tensor-bound and
+    // memory-bound work overlap. Back to back against equal shares of per-tile costs alone (us): 256
+    // captures of up to 2^22 samples 890 -> 813, 224 of up to 2^20 264 -> 224, 200 of up to 2^18 129 ->
+    // 108, 70 of up to 2^18 67 -> 46 (with the window tiles' tap matrices in tensor memory). Letting
+    // each phase start over at the first block, to fill what the long-filter tiles leave there, was
+    // faster for some batches (64 of up to 2^21 134 -> 127, before the second limit) and slower for
+    // others (256: 803 -> 825).
+    const int most = std::min({sms, kBatchCtas, units});
+    std::vector<int> tiles[kPhases];
+    double longest = 1.01 * all_us;   // fits one block
     double low = 0.0;
-    double high = 0.0;
-    for (const Run& run : line) {
-        high += run.tiles * run.cost.tile + run.cost.start + kPhaseUs[run.phase];
-    }
     for (int step = 0; step < 40; ++step) {
-        const double mid = 0.5 * (low + high);
-        (cut_line(line, mid, grid, &ends) ? high : low) = mid;
+        const double mid = 0.5 * (low + longest);
+        (deal(runs, mid, mid, most, tiles) ? longest : low) = mid;
     }
-    if (!cut_line(line, high, grid, &ends)) {
+    double rest = longest;
+    low = 0.0;
+    for (int step = 0; step < 40; ++step) {
+        const double mid = 0.5 * (low + rest);
+        (deal(runs, longest, mid, most, tiles) ? rest : low) = mid;
+    }
+    if (!deal(runs, longest, rest, most, tiles)) {
         delete plan;
-        return cudaErrorInvalidValue;   // not reached: the whole line fits one piece
+        return cudaErrorInvalidValue;   // not reached: these limits have been dealt
     }
-    grid = static_cast<int>(ends.size());
-    std::vector<int> cta_item(grid + 1), cta_plain(grid + 1);
-    std::vector<int> cta_win[tcw::kCMax];
-    for (auto& cw : cta_win) {
-        cw.assign(grid + 1, 0);
-    }
-    for (int b = 1; b <= grid; ++b) {
-        // Units of phase ph in the pieces before block b.
-        auto in_phase = [&](int ph) {
-            return std::min(std::max(ends[b - 1] - base[ph], 0), base[ph + 1] - base[ph]);
-        };
-        cta_item[b] = in_phase(0);
-        for (int ci = 0; ci < tcw::kCMax; ++ci) {
-            cta_win[ci][b] = in_phase(ci + 1);
+    int grid = 0;   // blocks with work: the first ones
+    for (int b = 0; b < most; ++b) {
+        for (const auto& list : tiles) {
+            grid = list[b] > 0 ? b + 1 : grid;
         }
-        cta_plain[b] = in_phase(kPhases - 1);
     }
+    // First tile of each block in each phase.
+    std::vector<int> first[kPhases];
+    for (int ph = 0; ph < kPhases; ++ph) {
+        first[ph].assign(grid + 1, 0);
+        for (int b = 0; b < grid; ++b) {
+            first[ph][b + 1] = first[ph][b] + tiles[ph][b];
+        }
+    }
+    const std::vector<int>& cta_item = first[0];
+    const std::vector<int>* cta_win = &first[1];
+    const std::vector<int>& cta_plain = first[kPhases - 1];
 
     // One device buffer: capture table, tensor maps (128-byte aligned), block ranges, plain
     // captures.

@@ -1,14 +1,15 @@
-// The resident-window tensor-core FIR pipeline (2 to 385 taps) as a device-side template, run by
+// The resident-window tensor-core FIR pipeline (2 to 1025 taps) as a device-side template, run by
 // the single-capture kernel (fir_tc_win.cu) and by the batch kernel's window phase
 // (fir_batch.cu). The algorithm, its roles and their measured costs are described in
-// fir_tc_win.cu; this header holds the pipeline and the two ways it finds its tiles:
+// fir_tc_win.cu; this header holds the pipeline and the three ways it finds its tiles:
 //  * TcwSingleSrc: one capture, tile k of a block = blockIdx.x + k gridDim.x;
 //  * TcwSharedSrc: several captures with one tap set, tiles of all of them dealt out the same way;
 //  * TcwListSrc: a contiguous range of (capture, tile) work items, captures in increasing order,
 //    each with its own taps, length and tensor map (in global memory). The tap strip is then
 //    rebuilt per capture by the scan warps, into one of two strip slots or into the only one
 //    (kStrips), after the MMA warp's `strip_free` commit for the capture that used the slot
-//    last, and published with `strip_ready`; the scan warps publish the capture's first tile
+//    last, and published with `strip_ready`, from where the drain warps take the tap matrices that
+//    tensor memory holds (`taps_ready`); the scan warps publish the capture's first tile
 //    scale before they wait for the slot, and the drain's tap scale travels with each tile's
 //    sample scale.
 #pragma once
@@ -98,6 +99,7 @@ struct Ctrl {
     unsigned long long patched;          // the partial last block written into its window row
     unsigned long long strip_ready[2];   // a strip slot built (every scan warp)
     unsigned long long strip_free[2];    // the MMAs reading a strip slot done (tcgen05.commit)
+    unsigned long long taps_ready;       // tap matrices in tensor memory (every drain warp)
     unsigned long long teardown;
     int abort;
     uint32_t pmax[2][kScanWarps];
@@ -285,6 +287,7 @@ __device__ __forceinline__ void tcw_init(Ctrl& ctl)
         mbar_init(smem_u32(&ctl.sready[i]), 1);
     }
     mbar_init(smem_u32(&ctl.patched), kScanWarps);
+    mbar_init(smem_u32(&ctl.taps_ready), kDrainWarps);
     mbar_init(smem_u32(&ctl.teardown), 1);
     ctl.abort = 0;
     ctl.tap_max = 0;
@@ -311,11 +314,11 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
     constexpr uint32_t kIdesc = idesc_f16(kB, 2 * NB);
     constexpr uint32_t kN = 2 * NB;           // columns of an accumulator
     constexpr uint32_t kXCol = 2 * kN;        // first column of X0
-    // Tap matrices in tensor memory (one tap set; fir_tc_win.cu gives the reason): chunk c's eight
+    // Tap matrices in tensor memory (fir_tc_win.cu gives the reason): chunk c's eight
     // K-steps take 64 columns per split, the high split's chunks first, then the low split's, as
     // far as the columns go. The other MMAs read the strip in shared memory.
     constexpr int kChunkCols = 8 * kSteps;
-    constexpr int kRoom = kMulti || (NB <= 16 && C <= 2)
+    constexpr int kRoom = NB <= 16 && C <= 2
                               ? 0
                               : static_cast<int>(kTmemCols - 4 * kN) / kChunkCols;
     constexpr int kHiChunks = kRoom < C + 1 ? kRoom : C + 1;
@@ -486,10 +489,6 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
         const uint32_t stage_units = lay.stage >> 4;
         const uint32_t split_units = lay.split >> 4;
         bool stop = false;
-        if constexpr (kRoom > 0) {
-            asm volatile("bar.sync 1, %0;" ::"n"((kDrainWarps + 1) * 32) : "memory");
-            fence_after();   // the drain warps' tap matrices
-        }
         int u = 0;     // K-steps issued (block-wide numbering)
         int g = 0;     // H groups issued
         TcwCursor cur;
@@ -512,6 +511,13 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
                                            fault, kFaultStageFull, abort)) {
                         break;
                     }
+                }
+                if (kRoom > 0 && (kMulti || occ == 0)) {
+                    if (!mbar_wait_bounded(smem_u32(&ctl.taps_ready), occ & 1, fault,
+                                           kFaultStageFull, abort)) {
+                        break;
+                    }
+                    fence_after();
                 }
                 const int zero_top = C * kB - src.capture(cur.idx).num_taps - 15;
                 st_cmax = zero_top < 0 ? 0 : zero_top / 16 + 1;
@@ -715,9 +721,19 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
         const int r = kB - 1 - (quarter * 32 + lane);          // output row of this TMEM lane
         const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) +
                                    static_cast<uint32_t>(half * NB);
-        if constexpr (kRoom > 0) {
-            // The tap matrices, while the first tile is converted. Matrix (c, st), row m (lane m):
-            // strip elements 16 C + 2 st - 16 c + m / 8 and the next, row m % 8 of each.
+        // The tap matrices of capture number occ of this block, once its strip is built: the first
+        // one's while the first tile is converted, a later one's as soon as the MMAs of the capture
+        // before it are done, before its last tile is drained. Matrix (c, st), row m (lane m): strip
+        // elements 16 C + 2 st - 16 c + m / 8 and the next, row m % 8 of each.
+        auto store_taps = [&](int occ) {
+            if constexpr (kMulti) {
+                if (!mbar_wait_bounded(smem_u32(&ctl.strip_ready[strip_slot(occ)]),
+                                       strip_use(occ) & 1, fault, kFaultStageFull, abort)) {
+                    return false;
+                }
+                fence_after();
+            }
+            const int slot = kMulti ? strip_slot(occ) : 0;
             const int m = quarter * 32 + lane;
             const uint32_t row_off = static_cast<uint32_t>(16 * C + m / 8) * 128u +
                                      static_cast<uint32_t>(m % 8) * 16u;
@@ -727,7 +743,7 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
             for (int i = half; i < kMatrices; i += kDrainWarps / 4) {
                 const bool hi = i < kHiChunks * kSteps;
                 const int j = hi ? i : i - kHiChunks * kSteps;   // 8 c + st
-                const uint32_t from = (hi ? strip_hi(0) : strip_lo(0)) + row_off +
+                const uint32_t from = (hi ? strip_hi(slot) : strip_lo(slot)) + row_off +
                                       static_cast<uint32_t>(2 * (j % kSteps)) * 128u -
                                       static_cast<uint32_t>(16 * (j / kSteps)) * 128u;
                 const float4 e0 = lds128(from);
@@ -740,7 +756,31 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
             }
             tmem_wait_st();
             fence_before();
-            asm volatile("bar.arrive 1, %0;" ::"n"((kDrainWarps + 1) * 32) : "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(smem_u32(&ctl.taps_ready));
+            }
+            return true;
+        };
+        int taps_occ = 0;   // captures whose matrices are stored, less one
+        // After the accumulators of tile k are complete: the next tile's capture, if another.
+        auto next_taps = [&](int k, const TcwCursor& cur) {
+            if constexpr (kMulti && kRoom > 0) {
+                if (k + 1 < my_tiles) {
+                    TcwCursor next = cur;
+                    long long tn;
+                    src.locate(k + 1, next, tn);
+                    if (next.idx != cur.idx) {
+                        return store_taps(++taps_occ);
+                    }
+                }
+            }
+            return true;
+        };
+        if constexpr (kRoom > 0) {
+            if (my_tiles > 0) {
+                store_taps(0);   // (a give-up shows in *abort)
+            }
         }
         float acc[groups > 1 ? NB : 1];
 #pragma unroll
@@ -788,7 +828,8 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
                 if (!mbar_wait_bounded(smem_u32(&ctl.xfull[k & 1]), (k >> 1) & 1, fault,
                                        kFaultAccumFull, abort) ||
                     !mbar_wait_bounded(smem_u32(&ctl.sready[k % kScales]), (k / kScales) & 1,
-                                       fault, kFaultScale, abort)) {
+                                       fault, kFaultScale, abort) ||
+                    !next_taps(k, cur)) {
                     break;
                 }
                 fence_after();
@@ -860,7 +901,8 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
                 !mbar_wait_bounded(smem_u32(&ctl.xfull[k & 1]), (k >> 1) & 1, fault,
                                    kFaultAccumFull, abort) ||
                 !mbar_wait_bounded(smem_u32(&ctl.sready[k % kScales]), (k / kScales) & 1, fault,
-                                   kFaultScale, abort)) {
+                                   kFaultScale, abort) ||
+                !next_taps(k, cur)) {
                 break;
             }
             fence_after();
@@ -1030,6 +1072,7 @@ __device__ __forceinline__ void tcw_release(Ctrl& ctl)
         inval(&ctl.sready[i]);
     }
     inval(&ctl.patched);
+    inval(&ctl.taps_ready);
     inval(&ctl.teardown);
 }
 
