@@ -146,6 +146,7 @@ chan_dft_kernel(const float2* __restrict__ u, const uint4* __restrict__ image,
     if (warp == kMmaWarp) {
         tmem_alloc(smem_u32(&ctl.tmem_base), kTmemCols);
     }
+    __syncthreads();   // tensor memory is held before the next kernel is let in (allow_next)
     wait_for_stream();
     allow_next();
     {

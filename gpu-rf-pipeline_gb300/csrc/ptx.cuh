@@ -188,8 +188,12 @@ __device__ __forceinline__ void wait_for_stream()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Lets the next kernel of the stream be scheduled once every block of this one has come here.
-// After wait_for_stream(), so that no more than two kernels of a stream are ever in flight.
+// Lets the next kernel of the stream be scheduled once every block of this one has come here (a
+// block has come here with its first warp). After wait_for_stream(), so that no more than two
+// kernels of a stream are ever in flight; and in a kernel that allocates tensor memory after a block
+// barrier behind the allocation: a block of the next kernel allocates before its own wait and holds
+// its columns until this kernel has completed, so a block of this one that had not allocated yet
+// could wait for them for ever.
 __device__ __forceinline__ void allow_next()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
