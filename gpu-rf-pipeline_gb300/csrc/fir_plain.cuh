@@ -11,12 +11,15 @@ constexpr int kPlainOutputsPerThread = 9;
 constexpr int kPlainTileOutputs = kPlainThreads * kPlainOutputsPerThread;  // 2304
 constexpr int kMaxTaps = 8192;  // the project's constant-bank capacity (src/fir.cu:208)
 
-// Captures sharing one tap set, passed by value as one kernel argument (64 * 24 bytes).
+// Captures sharing one tap set, passed by value as one kernel argument: blocks take the captures'
+// tiles in order (tile0[c] = first block of capture c, filled in by the launch).
 constexpr int kPlainBatchMax = 64;
 struct PlainBatch {
     const void* x[kPlainBatchMax];
     void* y[kPlainBatchMax];
     long long num_samples[kPlainBatchMax];
+    int tile0[kPlainBatchMax + 1];
+    int count;
 };
 
 // Captures with their own taps, one launch for all: blocks take the captures' tiles in order
@@ -34,8 +37,8 @@ struct PlainCaps {
 
 cudaError_t fir_plain_launch(const void* x, const float* taps, void* y, long long n,
                              int num_taps, cudaStream_t stream);
-cudaError_t fir_plain_batched_launch(const PlainBatch& batch, int count, const float* taps,
-                                     int num_taps, cudaStream_t stream);
+cudaError_t fir_plain_batched_launch(PlainBatch& batch, const float* taps, int num_taps,
+                                     cudaStream_t stream);
 // The FIR of integer I/Q input decoded in the load stage: format 1 = ci16 (components x / 32768),
 // 2 = ci8 (x / 128), 0 = cf32 (fir_plain_launch). Same bits as decoding first.
 cudaError_t fir_plain_launch_format(int format, const void* x, const float* taps, void* y,

@@ -440,13 +440,13 @@ int rfx_fir_batched_device(int impl, const void* const* x, void* const* y,
     for (int first = 0; first < count; first += rfx::kPlainBatchMax) {
         const int chunk = std::min(count - first, rfx::kPlainBatchMax);
         rfx::PlainBatch batch{};
+        batch.count = chunk;
         for (int c = 0; c < chunk; ++c) {
             batch.x[c] = x[first + c];
             batch.y[c] = y[first + c];
             batch.num_samples[c] = num_samples[first + c];
         }
-        const cudaError_t err =
-            rfx::fir_plain_batched_launch(batch, chunk, taps, num_taps, stream);
+        const cudaError_t err = rfx::fir_plain_batched_launch(batch, taps, num_taps, stream);
         if (err != cudaSuccess) {
             return cuda_fail(err, "fir_plain_batched_launch");
         }
