@@ -112,11 +112,19 @@ static cudaError_t ensure_smem_attr(const void* fn, size_t bytes)
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
 }
 
-// Shared memory for a launch of `blocks` tiles, `fit` of which fit an SM, and the function's
-// opt-in to it.
-static cudaError_t spread_tiles(const void* fn, long long blocks, int sms, int fit, size_t* bytes)
+// Blocks of `threads` threads (1024 to an SM: the kernels' launch bounds) and `bytes` of shared memory
+// that fit an SM.
+static int tiles_that_fit(int threads, size_t bytes)
 {
-    *bytes = even_spread_smem(*bytes, blocks, sms, fit);
+    const int by_smem = static_cast<int>(kSmemPerSm / (bytes + kSmemPerBlock));
+    return by_smem < 1024 / threads ? by_smem : 1024 / threads;
+}
+
+// Shared memory for a launch of `blocks` tiles and the function's opt-in to it.
+static cudaError_t spread_tiles(const void* fn, long long blocks, int sms, int threads,
+                                size_t* bytes)
+{
+    *bytes = even_spread_smem(*bytes, blocks, sms, tiles_that_fit(threads, *bytes));
     return ensure_smem_attr(fn, *bytes);
 }
 
@@ -142,10 +150,12 @@ struct TileShape {
 // with staging. Measured, 1025 taps (us): 4096 samples 8.6 (3 outputs) against 25.5 for the tile of
 // 256 threads and 9 outputs that every call took, 65536 samples 11.5 (5) against 25.4, 2^18 samples
 // 20.9 (7) against 25.6; 63 taps: 10007 samples 2.4 against 4.0, 2^24 75.6 (9 outputs, 128 threads)
-// against 78.1.
+// against 78.1. Long filters take so much shared memory that one or two blocks fill an SM: a warp is
+// alone on its scheduler then, however many tiles wait, and the larger block is the better one (2^22
+// samples of cf32, 8192 taps 2185 us with 256 threads of 9 outputs against 2371 with 128).
 // tiles_of(outputs): the launch's tiles of that many outputs each.
 template <class Tiles>
-static TileShape tile_shape(Tiles tiles_of, int num_taps, int sms)
+static TileShape tile_shape(Tiles tiles_of, int num_taps, int fmt, int sms)
 {
     struct Candidate {
         TileShape shape;
@@ -156,6 +166,7 @@ static TileShape tile_shape(Tiles tiles_of, int num_taps, int sms)
     };
     static constexpr Candidate kCandidates[] = {
         {{128, 9}, 23.3, 26.0, 780.0, 2500.0},
+        {{256, 9}, 23.3, 26.0, 780.0, 3100.0},
         {{256, 7}, 18.9, 18.9, 620.0, 3100.0},
         {{128, 5}, 15.2, 18.6, 480.0, 1400.0},
         {{128, 3}, 12.5, 12.5, 460.0, 1500.0},
@@ -166,7 +177,12 @@ static TileShape tile_shape(Tiles tiles_of, int num_taps, int sms)
         const long long tile = static_cast<long long>(c.shape.threads) * c.shape.outputs;
         const long long per_sm = (tiles_of(tile) + sms - 1) / sms;
         const double w = static_cast<double>(per_sm) * c.shape.threads / 128.0;
-        const double tap = w > 1.0 ? w * c.per_tap : c.alone;
+        const long long fit = tiles_that_fit(
+            c.shape.threads, plain_layout(num_taps, fmt, static_cast<int>(tile)).bytes);
+        const double live = static_cast<double>(per_sm < fit ? per_sm : fit) * c.shape.threads / 128.0;
+        // Fewer than four warps on a scheduler, though more wait: 2 % of staging in the open.
+        const double open = per_sm > fit && live < 4.0 ? 1.02 : 1.0;
+        const double tap = w * (live > 1.0 ? open * c.per_tap : c.alone);
         double cycles = num_taps * tap;
         cycles = cycles > w * c.least ? cycles : w * c.least;
         cycles = cycles > c.floor_cycles ? cycles : c.floor_cycles;
@@ -183,6 +199,9 @@ template <class Run>
 static cudaError_t with_shape(TileShape shape, Run run)
 {
     using std::integral_constant;
+    if (shape.threads == 256 && shape.outputs == 9) {
+        return run(integral_constant<int, 9>{}, integral_constant<int, 256>{});
+    }
     switch (shape.outputs) {
     case 3: return run(integral_constant<int, 3>{}, integral_constant<int, 128>{});
     case 5: return run(integral_constant<int, 5>{}, integral_constant<int, 128>{});
@@ -204,14 +223,14 @@ static cudaError_t launch_plain(const void* x, const float* taps, void* y, long 
         return err;
     }
     auto tiles_of = [n](long long tile) { return (n + tile - 1) / tile; };
-    return with_shape(tile_shape(tiles_of, num_taps, sms), [&](auto r, auto t) {
+    return with_shape(tile_shape(tiles_of, num_taps, kFmt, sms), [&](auto r, auto t) {
         constexpr int R = decltype(r)::value;
         constexpr int T = decltype(t)::value;
         auto kernel = fir_plain_kernel<kFmt, R, T>;
         const long long tiles = tiles_of(T * R);
         size_t bytes = plain_layout(num_taps, kFmt, T * R).bytes;
         const cudaError_t e =
-            spread_tiles(reinterpret_cast<const void*>(kernel), tiles, sms, 1024 / T, &bytes);
+            spread_tiles(reinterpret_cast<const void*>(kernel), tiles, sms, T, &bytes);
         if (e != cudaSuccess) {
             return e;
         }
@@ -246,7 +265,7 @@ cudaError_t fir_plain_batched_launch(PlainBatch& batch, const float* taps, int n
     if (err != cudaSuccess) {
         return err;
     }
-    return with_shape(tile_shape(tiles_of, num_taps, sms), [&](auto r, auto t) {
+    return with_shape(tile_shape(tiles_of, num_taps, 0, sms), [&](auto r, auto t) {
         constexpr int R = decltype(r)::value;
         constexpr int T = decltype(t)::value;
         auto kernel = fir_plain_batched_kernel<R, T>;
@@ -258,7 +277,7 @@ cudaError_t fir_plain_batched_launch(PlainBatch& batch, const float* taps, int n
         }
         size_t bytes = plain_layout(num_taps, 0, T * R).bytes;
         const cudaError_t e =
-            spread_tiles(reinterpret_cast<const void*>(kernel), tiles, sms, 1024 / T, &bytes);
+            spread_tiles(reinterpret_cast<const void*>(kernel), tiles, sms, T, &bytes);
         if (e != cudaSuccess) {
             return e;
         }
@@ -293,7 +312,8 @@ cudaError_t fir_plain_caps_launch(const PlainCaps& caps, cudaStream_t stream)
         return err;
     }
     size_t bytes = plain_layout(kmax).bytes;
-    err = spread_tiles(reinterpret_cast<const void*>(fir_plain_caps_kernel), tiles, sms, 4, &bytes);
+    err = spread_tiles(reinterpret_cast<const void*>(fir_plain_caps_kernel), tiles, sms, kThreads,
+                       &bytes);
     if (err != cudaSuccess) {
         return err;
     }

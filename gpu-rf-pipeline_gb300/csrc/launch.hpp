@@ -33,6 +33,9 @@ cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, 
     return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
+constexpr size_t kSmemPerSm = 228u * 1024u;    // shared memory of an SM
+constexpr size_t kSmemPerBlock = 1024u;        // of which the system takes this much per block
+
 // Dynamic shared memory to ask for so that no multiprocessor takes more than its share,
 // ceil(blocks / sms), of a launch smaller than one full wave (`bytes` needed, `fit` blocks fit an
 // SM). Launched in the ordinary way blocks spread evenly; while the kernel before still holds its
@@ -44,9 +47,7 @@ inline size_t even_spread_smem(size_t bytes, long long blocks, int sms, int fit)
     if (share >= fit || 2 * blocks <= sms) {
         return bytes;   // a full wave, or few enough that idle multiprocessors remain
     }
-    constexpr size_t kPerSm = 228u * 1024u;    // shared memory of an SM
-    constexpr size_t kPerBlock = 1024u;        // of which the system takes this much per block
-    const size_t more_than = kPerSm / static_cast<size_t>(share + 1) - kPerBlock;
+    const size_t more_than = kSmemPerSm / static_cast<size_t>(share + 1) - kSmemPerBlock;
     const size_t padded = (more_than / 128u + 1u) * 128u;   // share + 1 blocks do not fit
     return bytes > padded ? bytes : padded;
 }
