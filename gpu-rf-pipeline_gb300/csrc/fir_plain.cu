@@ -44,7 +44,11 @@ fir_plain_kernel(const void* __restrict__ x, const float* __restrict__ taps,
     plain_block_tile<kFmt, R, T>(x, taps, y, n, num_taps, blockIdx.x, smem);
 }
 
-// The capture c that block `block` works on: the last with tile0[c] <= block.
+// The capture c that block `block` works on: the last with tile0[c] <= block. Through a warp
+// reduction, so that the compiler knows it to be the same on every lane and keeps the capture's
+// fields and what follows from them in uniform registers: 2^22 samples, 700 taps 188.3 us, as for one
+// capture in the kernel's parameters, against 198 with the search's own result (more register bank
+// conflicts on the packed multiply-adds).
 template <class Captures>
 __device__ __forceinline__ int capture_of(const Captures& captures, int block)
 {
@@ -58,7 +62,7 @@ __device__ __forceinline__ int capture_of(const Captures& captures, int block)
             hi = mid;
         }
     }
-    return lo;
+    return static_cast<int>(__reduce_max_sync(0xFFFFFFFFu, static_cast<unsigned>(lo)));
 }
 
 // Several captures sharing one tap set: block b takes tile b - tile0[c] of the capture c whose tiles
