@@ -451,12 +451,8 @@ cudaError_t launch(const void* x, const float* taps, void* out, long long frames
     const int guard = kR * (PG + 1);
     const size_t bytes = even_spread_smem(C::kBytes, blocks, sms, C::kBlocks);
     auto kernel = chan_fused_kernel<M, PG, kFmt, kMag>;
-    if (bytes > 48u * 1024u) {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(bytes));
-        if (err != cudaSuccess) {
-            return err;
-        }
+    if ((err = opt_in_smem(kernel, bytes)) != cudaSuccess) {
+        return err;
     }
     return launch_overlapped(kernel, blocks, C::kThreads, bytes, stream, x, taps, out, n,
                              static_cast<int>(frames), num_taps, static_cast<int>(seg), guard,

@@ -582,12 +582,9 @@ cudaError_t chan_branch_launch(const void* x, const float* taps, void* u, long l
     const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
     float2* uo = static_cast<float2*>(u);
     auto run = [&](auto kernel, size_t bytes) -> cudaError_t {
-        if (bytes > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(
-                kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-            if (e != cudaSuccess) {
-                return e;
-            }
+        const cudaError_t e = opt_in_smem(kernel, bytes);
+        if (e != cudaSuccess) {
+            return e;
         }
         return launch_overlapped(kernel, grid, kBranchThreads, bytes, stream, x, taps, uo, n, frames,
                                  channels, num_taps, w, guard_frames);

@@ -666,10 +666,7 @@ static cudaError_t launch_chan(const void* x, const float* taps, const void* twi
     if (attr.maxThreadsPerBlock < kThreads) {
         return cudaErrorLaunchOutOfResources;
     }
-    err = cudaFuncSetAttribute(chan_tc_kernel<kTapsSmem, kMag, kFmt>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(bytes));
-    if (err != cudaSuccess) {
+    if ((err = opt_in_smem(chan_tc_kernel<kTapsSmem, kMag, kFmt>, bytes)) != cudaSuccess) {
         return err;
     }
     // x viewed as rows of 128 components (one frame of 64 samples), full frames only; boxes of

@@ -35,6 +35,7 @@
 #include "fir_tc.cuh"
 #include "fir_plain.cuh"
 #include "fir_plain_tile.cuh"
+#include "launch.hpp"
 #include "tc_common.cuh"
 #include "tmap.hpp"
 #include "tuning.hpp"
@@ -1104,9 +1105,7 @@ cudaError_t launch_batch(const BatchParams& params, int grid, const Layout& lay,
                          cudaStream_t stream)
 {
     const uint32_t bytes = lay.bytes > 120u * 1024u ? lay.bytes : 120u * 1024u;
-    cudaError_t err = cudaFuncSetAttribute(fir_batch_kernel<S>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(bytes));
+    const cudaError_t err = opt_in_smem(fir_batch_kernel<S>, bytes);
     if (err != cudaSuccess) {
         return err;
     }
@@ -1608,8 +1607,7 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
     const void* fn = plan->stages == 6   ? reinterpret_cast<const void*>(fir_batch_list_kernel<6>)
                      : plan->stages == 4 ? reinterpret_cast<const void*>(fir_batch_list_kernel<4>)
                                          : reinterpret_cast<const void*>(fir_batch_list_kernel<2>);
-    if ((err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(plan->smem))) != cudaSuccess) {
+    if ((err = opt_in_smem(fn, plan->smem)) != cudaSuccess) {
         fir_batch_plan_free(plan);
         return err;
     }

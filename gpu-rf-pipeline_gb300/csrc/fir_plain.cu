@@ -96,26 +96,6 @@ fir_plain_caps_kernel(const __grid_constant__ PlainCaps caps)
                      caps.num_taps[c], block - caps.tile0[c], smem);
 }
 
-static cudaError_t ensure_smem_attr(const void* fn, size_t bytes)
-{
-    // The opt-in limit only has to be raised once per function and size class; raising it to
-    // the device maximum once covers every tap count.
-    if (bytes <= 48 * 1024) {
-        return cudaSuccess;
-    }
-    int device = 0;
-    cudaError_t err = cudaGetDevice(&device);
-    if (err != cudaSuccess) {
-        return err;
-    }
-    int optin = 0;
-    err = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    if (err != cudaSuccess) {
-        return err;
-    }
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-}
-
 // Blocks of `threads` threads (1024 to an SM: the kernels' launch bounds) and `bytes` of shared memory
 // that fit an SM.
 static int tiles_that_fit(int threads, size_t bytes)
@@ -129,7 +109,7 @@ static cudaError_t spread_tiles(const void* fn, long long blocks, int sms, int t
                                 size_t* bytes)
 {
     *bytes = even_spread_smem(*bytes, blocks, sms, tiles_that_fit(threads, *bytes));
-    return ensure_smem_attr(fn, *bytes);
+    return opt_in_smem(fn, *bytes);
 }
 
 static cudaError_t sm_count(int* sms)

@@ -773,9 +773,7 @@ static cudaError_t launch_stages(int fmt, const void* x, const float* taps, void
     if (attr.maxThreadsPerBlock < kThreads) {
         return cudaErrorLaunchOutOfResources;
     }
-    err = cudaFuncSetAttribute(fir_tc_kernel<S, kInt>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(bytes));
-    if (err != cudaSuccess) {
+    if ((err = opt_in_smem(fir_tc_kernel<S, kInt>, bytes)) != cudaSuccess) {
         return err;
     }
     // x viewed as rows of 256 components (one 128-sample block per row), full blocks only;

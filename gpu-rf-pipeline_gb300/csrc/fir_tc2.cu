@@ -32,6 +32,7 @@
 // each on the even CTA's mbarriers; the MMA commits arrive on both CTAs' mbarriers
 // (multicast). Every wait is bounded in time.
 #include "fir_tc2.cuh"
+#include "launch.hpp"
 #include "tc_common.cuh"
 #include "tc_pair.cuh"
 #include "tmap.hpp"
@@ -771,9 +772,7 @@ static cudaError_t launch_pair(const void* x, const float* taps, void* y, long l
     if (attr.maxThreadsPerBlock < kThreads) {
         return cudaErrorLaunchOutOfResources;
     }
-    err = cudaFuncSetAttribute(fir_tc2_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(bytes));
-    if (err != cudaSuccess) {
+    if ((err = opt_in_smem(fir_tc2_kernel<S>, bytes)) != cudaSuccess) {
         return err;
     }
     CUtensorMap map;

@@ -33,6 +33,35 @@ cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, 
     return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
+// Lets launches of `kernel` (which has no static shared memory) ask for `bytes` of dynamic shared
+// memory. The limit belongs to the function, not to the launch: set to what one call needs, it fails
+// a call of another thread, or a plan made before, that needs more and launches after it. So always
+// the device's limit.
+inline cudaError_t opt_in_smem(const void* kernel, size_t bytes)
+{
+    if (bytes <= 48u * 1024u) {
+        return cudaSuccess;
+    }
+    int device = 0;
+    int limit = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err == cudaSuccess) {
+        err = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    }
+    if (err != cudaSuccess) {
+        return err;
+    }
+    return bytes > static_cast<size_t>(limit)
+               ? cudaErrorInvalidValue
+               : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+}
+
+template <class... Params>
+cudaError_t opt_in_smem(void (*kernel)(Params...), size_t bytes)
+{
+    return opt_in_smem(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 constexpr size_t kSmemPerSm = 228u * 1024u;    // shared memory of an SM
 constexpr size_t kSmemPerBlock = 1024u;        // of which the system takes this much per block
 
