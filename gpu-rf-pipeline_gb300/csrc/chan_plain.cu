@@ -520,7 +520,7 @@ static cudaError_t ring_launch(const void* x, const float* taps, float2* u, long
     seg_frames = (seg_frames + kR - 1) / kR * kR;
     const long long segs = (frames + seg_frames - 1) / seg_frames;
     const long long bx = (segs + per_block - 1) / per_block;
-    if (bx > 0x7FFFFFFFLL || gy > 65535) {
+    if (bx > 0x7FFFFFFFLL) {
         return cudaErrorInvalidConfiguration;
     }
     const int guard_frames = kR * (groups + 1);
@@ -544,7 +544,9 @@ cudaError_t chan_branch_launch(const void* x, const float* taps, void* u, long l
     }
     {
         const long long n = (frames - 1) * static_cast<long long>(channels) + 1;
-        if (num_taps <= 4LL * kR * channels) {
+        // (The grid has room for 65535 rows of blocks: of 128 branches each in the ring form, of 256
+        // in the one below.)
+        if (num_taps <= 4LL * kR * channels && channels <= 65535LL * kRingThreads) {
             return ring_launch(x, taps, static_cast<float2*>(u), n, frames, channels, num_taps,
                                stream, format);
         }
