@@ -944,9 +944,19 @@ __device__ __forceinline__ void batch_plain_tiles(const BatchView& p, int t0, in
     const int gtid = static_cast<int>(threadIdx.x) % kPlainThreads;
     unsigned char* region = smem + 1024 + static_cast<uint32_t>(group) * p.plain_region;
     const PlainGroupSync sync{static_cast<uint32_t>(2 + group)};
+    // The capture of the group's first tile by binary search (a scan from the list's start, dependent
+    // loads all, took 25 us behind 152 captures); from there the tiles only move forward.
+    int c = 0;
+    for (int hi = p.pcount - 1; c < hi;) {
+        const int mid = (c + hi + 1) >> 1;
+        if (p.pcap[mid].tile0 <= t0 + group) {
+            c = mid;
+        } else {
+            hi = mid - 1;
+        }
+    }
     if (p.plain_region >= 2 * p.plain_slot) {
         // Two slots: each tile's copy overlaps the previous tile's computation.
-        int c = 0;
         auto source = [&](int i) {
             const int t = t0 + group + i * p.plain_groups;
             while (c + 1 < p.pcount && p.pcap[c + 1].tile0 <= t) {
@@ -964,7 +974,6 @@ __device__ __forceinline__ void batch_plain_tiles(const BatchView& p, int t0, in
     }
     uint32_t phase = 0;
     bool init = true;
-    int c = 0;
     for (int t = t0 + group; t < t1; t += p.plain_groups) {
         while (c + 1 < p.pcount && p.pcap[c + 1].tile0 <= t) {
             ++c;
@@ -1231,9 +1240,11 @@ namespace {
 // taps (C = 4) and 16.5 at 1025 (C = 8), 9.9 per capture; a window tile of 48 blocks 2.11, 2.16 and
 // 2.20 at 31, 63 and 127 taps (C = 1), 2.83 at 255 (C = 2), 2.5 and 4.1 per capture, 4.1 and 5.4 per
 // phase (2.39, 2.46, 2.65 and 3.39 a tile before their tap matrices were in tensor memory); C = 3
-// scaled from single captures. Plain
-// tiles of 2304 outputs (batch plans of one tap count): 1.66, 2.27, 3.90, 6.54, 12.6 and 24.7 at 31,
-// 63, 127, 255, 511 and 1025 taps.
+// scaled from single captures. Plain tiles of 2304 outputs: 1.66, 2.27, 3.90, 6.54, 12.6 and 24.7 at
+// 31, 63, 127, 255, 511 and 1025 taps (batch plans of one tap count); at one tap, all that `auto`
+// leaves to them, 0.65 beside the windows' costs, by the time of plans of both (20 mixes of 16 to 200
+// captures): 1.0, a plan of one-tap captures alone, gave the windows too few blocks (16 captures of
+// 2^18 to 2^22 samples, three in four of one tap, the others of 255: 80.1 us; 66.2 now).
 struct Cost {
     double tile;
     double start;
@@ -1245,7 +1256,7 @@ Cost win_cost(int C, int num_taps)
            : C == 2 ? Cost{2.8, 4.1}
                     : Cost{3.5, 4.1};
 }
-Cost plain_cost(int num_taps) { return {1.0 + 0.0233 * static_cast<double>(num_taps), 0.0}; }
+Cost plain_cost(int num_taps) { return {0.65 + 0.0233 * static_cast<double>(num_taps), 0.7}; }
 // Phases in the order a block runs them: long-filter items, window items of C = 1, 2, 3, plain tiles.
 constexpr int kPhases = tcw::kCMax + 2;
 constexpr double kPhaseUs[kPhases] = {3.3, 4.1, 5.4, 5.4, 2.0};
