@@ -186,8 +186,8 @@ struct rfx_chan_plan {
     void* twiddles;       // tensor core: the DFT operand image, built once in FP64
     void* scratch;        // plain: channel outputs before their magnitude (first such call);
                           // tensor core, 1024 channels: the branch sums (made with the plan)
-    bool fused;           // RFX_CHAN_AUTO at 64 channels: the fused FP32 kernel, within the
-                          // limits of the tensor-core form's plans
+    bool fused;           // RFX_CHAN_AUTO at 64 channels: calls up to the plan's length that the
+                          // fused FP32 kernel takes run it; impl says what becomes of the others
 };
 
 extern "C" {
@@ -573,7 +573,7 @@ int rfx_chan_plan_create(int impl, int channels, int64_t max_samples, rfx_chan_p
     }
     auto* p = new rfx_chan_plan{impl, channels, rfx_channelize_frames(max_samples, channels), 0,
                                 false, nullptr, nullptr, fused};
-    if (fused) {
+    if (fused && impl == RFX_CHAN_TC) {
         *plan = p;   // its one kernel needs nothing beside the call's arguments
         return RFX_OK;
     }
@@ -722,6 +722,13 @@ int channelize_plan(rfx_chan_plan* plan, const void* x, const float* taps, void*
     if (!aligned16(x) || !aligned16(out)) {
         return fail(RFX_ERR_ALIGNMENT, "channelize: sample buffers must be 16-byte aligned");
     }
+    // (Less than a frame is left to impl: the tensor-core form's plans refuse it.)
+    if (plan->fused && frames <= plan->frames && num_samples >= plan->channels &&
+        rfx::chan_fused_supported(plan->channels, num_taps)) {
+        const cudaError_t err = rfx::chan_fused_launch(x, taps, out, frames, plan->channels,
+                                                       num_taps, magnitude, format, stream);
+        return err == cudaSuccess ? RFX_OK : cuda_fail(err, "chan_fused_launch");
+    }
     if (plan->impl == RFX_CHAN_TC) {
         if (frames > plan->frames) {
             return fail(RFX_ERR_INVALID, "channelize: plan made for up to %lld frames, call has "
@@ -740,12 +747,7 @@ int channelize_plan(rfx_chan_plan* plan, const void* x, const float* taps, void*
                         num_taps);
         }
         if (plan->fused) {
-            if (num_samples < plan->channels) {
-                return cuda_fail(cudaErrorInvalidValue, "chan_fused_launch");
-            }
-            const cudaError_t err = rfx::chan_fused_launch(
-                x, taps, out, frames, plan->channels, num_taps, magnitude, format, stream);
-            return err == cudaSuccess ? RFX_OK : cuda_fail(err, "chan_fused_launch");
+            return cuda_fail(cudaErrorInvalidValue, "chan_fused_launch");   // less than a frame
         }
         const cudaError_t err = rfx::chan_tc_launch(x, taps, plan->twiddles, out, num_samples,
                                                     num_taps, stream, magnitude, format);

@@ -303,17 +303,14 @@ TcConfig tuned_fir_tc_config(int num_taps, long long n)
 }
 
 // Built-in rule: at 64 channels the fused FP32 kernel (chan_fused.cuh) where the tensor-core form
-// stood; the plain form elsewhere, including 1024 channels, where the branch-sum kernel + cuFFT
+// stood (a tuned plain entry is the same kernel); the plain form elsewhere, including 1024 channels, where the branch-sum kernel + cuFFT
 // measured faster than the factored tensor-core DFT on GB300.
 int tuned_chan_impl(int channels, long long n, bool* fused)
 {
     ChanEntry e;
-    *fused = false;
-    if (lookup_chan(channels, n, &e)) {
-        return e.impl;
-    }
-    *fused = chan_tc_supported(channels, 1);
-    return *fused ? RFX_CHAN_TC : RFX_CHAN_PLAIN;
+    const bool tuned = lookup_chan(channels, n, &e);
+    *fused = chan_tc_supported(channels, 1) && !(tuned && e.impl == RFX_CHAN_TC);
+    return tuned ? e.impl : *fused ? RFX_CHAN_TC : RFX_CHAN_PLAIN;
 }
 
 }  // namespace rfx

@@ -72,7 +72,8 @@ typedef enum rfx_chan_impl {
     /* Chosen when the plan is made, from the tuned table (rfx_autotune_channelize) or the
      * built-in rule: the plain form, whose fused kernel at 64 channels runs in plans that take
      * what the tensor-core form's take (any call up to the plan's length, at least one whole
-     * frame, at most 2048 taps). */
+     * frame, at most 2048 taps). A tuned entry for the plain form adds what the plain form's plans
+     * take (calls of the plan's length, any tap count). */
     RFX_CHAN_AUTO = 2
 } rfx_chan_impl;
 
