@@ -16,7 +16,6 @@ struct TcConfig {
     int stages;       // operand ring depth cap (the largest that fits is used)
 };
 constexpr int kTcPairTile = 192;
-constexpr int kTcWindowTile = 48;   // the largest of the resident-window form
 
 // Whether a tile shape is the resident-window form's.
 constexpr bool is_window_tile(int tile_blocks)
@@ -49,10 +48,12 @@ cudaError_t fir_tcw_long_launch(int tile_blocks, int format, const void* x, cons
                                 void* y, long long n, int num_taps, cudaStream_t stream);
 cudaError_t fir_tcw_long_take_fault(unsigned int* code);
 // Up to kTcSharedMax captures sharing one tap set (cf32, each of at least 128 samples, none
-// touching what another writes) in one launch.
+// touching what another writes) in one launch, in tiles of `tile_blocks` blocks (0: by the built-in
+// rule over all their samples).
 constexpr int kTcSharedMax = 64;
-cudaError_t fir_tcw_shared_launch(const void* const* x, void* const* y, const int64_t* n, int count,
-                                  const float* taps, int num_taps, cudaStream_t stream);
+cudaError_t fir_tcw_shared_launch(int tile_blocks, const void* const* x, void* const* y,
+                                  const int64_t* n, int count, const float* taps, int num_taps,
+                                  cudaStream_t stream);
 // The tile the form takes for a capture of n samples by the built-in rule; 0 where the form for long
 // filters (fir_tc.cu) is the faster one.
 int fir_tcw_tile_blocks(int num_taps, long long n);

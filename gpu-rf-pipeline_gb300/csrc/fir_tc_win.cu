@@ -53,7 +53,8 @@
 
 namespace rfx {
 
-// Several cf32 captures with one tap set (each tile as in fir_tcw_kernel, so the same bits).
+// Several cf32 captures with one tap set, each tile as in fir_tcw_kernel: the same bits as the capture
+// alone where that takes the same tile (a tile's scale is taken over its own window).
 template <int C, int NB>
 __global__ void __launch_bounds__(tcw::kThreads, 1)
 fir_tcw_shared_kernel(const __grid_constant__ tcw::SharedCaptures list)
@@ -215,8 +216,9 @@ static cudaError_t launch_shared_reach(tcw::SharedCaptures& list, int num_taps, 
     }
 }
 
-cudaError_t fir_tcw_shared_launch(const void* const* x, void* const* y, const int64_t* n, int count,
-                                  const float* taps, int num_taps, cudaStream_t stream)
+cudaError_t fir_tcw_shared_launch(int tile_blocks, const void* const* x, void* const* y,
+                                  const int64_t* n, int count, const float* taps, int num_taps,
+                                  cudaStream_t stream)
 {
     int device = 0;
     int sms = 0;
@@ -243,12 +245,13 @@ cudaError_t fir_tcw_shared_launch(const void* const* x, void* const* y, const in
             tcw::WinCapture{x[c], static_cast<float2*>(y[c]), taps, n[c], num_taps, 0};
         total += n[c];
     }
-    switch (fir_tcw_tile_blocks(num_taps, total)) {
+    switch (tile_blocks != 0 ? tile_blocks : fir_tcw_tile_blocks(num_taps, total)) {
     case 8: return launch_shared_reach<8>(list, num_taps, sms, stream);
     case 16: return launch_shared_reach<16>(list, num_taps, sms, stream);
     case 24: return launch_shared_reach<24>(list, num_taps, sms, stream);
     case 32: return launch_shared_reach<32>(list, num_taps, sms, stream);
-    default: return launch_shared_reach<48>(list, num_taps, sms, stream);
+    case 48: return launch_shared_reach<48>(list, num_taps, sms, stream);
+    default: return cudaErrorInvalidValue;
     }
 }
 

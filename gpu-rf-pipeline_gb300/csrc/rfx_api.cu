@@ -395,19 +395,23 @@ int rfx_fir_batched_device(int impl, const void* const* x, void* const* y,
     const int resolved = resolve_fir_impl(impl, num_taps, longest);
     if (resolved == RFX_FIR_TC) {
         // Captures of the resident-window form share launches (8 captures of 2^16 to 2^18 samples,
-        // 127 taps: 8 launches 58.8 us, one 13.0). Those too short for a tensor map or tuned to
-        // another form take one each, and so do captures that read or overwrite what another of
-        // the call writes: they run one after another.
+        // 127 taps: 8 launches 58.8 us, one 13.0), in the tile that a tuned entry names for them or, by
+        // the built-in rule, the one for all their samples. Those too short for a tensor map or tuned
+        // to another form take one each; captures that are tuned to different tiles, or that read or
+        // overwrite what another of the call writes, run in launches one after another.
         const void* xs[rfx::kTcSharedMax];
         void* ys[rfx::kTcSharedMax];
         int64_t ns[rfx::kTcSharedMax];
         int shared = 0;
+        int shared_tile = 0;   // 0: by the built-in rule
         for (int c = 0; c <= count; ++c) {
+            rfx::TcConfig tuned{0, 0};
             const bool window =
                 c < count && num_samples[c] >= 128 && rfx::fir_tcw_supported(num_taps) &&
-                rfx::is_window_tile(
-                    rfx::tuned_fir_tc_config(num_taps, num_samples[c]).tile_blocks);
-            bool flush = c == count || shared == rfx::kTcSharedMax;
+                (!rfx::tuned_fir_tc_entry(num_taps, num_samples[c], &tuned) ||
+                 rfx::is_window_tile(tuned.tile_blocks));
+            bool flush = c == count || shared == rfx::kTcSharedMax ||
+                         (window && tuned.tile_blocks != shared_tile);
             for (int i = 0; i < shared && !flush; ++i) {
                 const size_t size = static_cast<size_t>(num_samples[c]) * 8u;
                 const size_t size_i = static_cast<size_t>(ns[i]) * 8u;
@@ -417,13 +421,15 @@ int rfx_fir_batched_device(int impl, const void* const* x, void* const* y,
             }
             if (flush && shared > 0) {
                 const cudaError_t err =
-                    rfx::fir_tcw_shared_launch(xs, ys, ns, shared, taps, num_taps, stream);
+                    rfx::fir_tcw_shared_launch(shared_tile, xs, ys, ns, shared, taps, num_taps,
+                                               stream);
                 if (err != cudaSuccess) {
                     return cuda_fail(err, "fir_tcw_shared_launch");
                 }
                 shared = 0;
             }
             if (window) {
+                shared_tile = tuned.tile_blocks;
                 xs[shared] = x[c];
                 ys[shared] = y[c];
                 ns[shared++] = num_samples[c];

@@ -291,11 +291,21 @@ int tuned_fir_batch_impl(int num_taps, long long n)
                : RFX_FIR_PLAIN;
 }
 
-TcConfig tuned_fir_tc_config(int num_taps, long long n)
+bool tuned_fir_tc_entry(int num_taps, long long n, TcConfig* config)
 {
     FirEntry e;
-    if (lookup_fir(num_taps, n, &e) && e.impl == RFX_FIR_TC) {
-        return e.config;
+    if (!lookup_fir(num_taps, n, &e) || e.impl != RFX_FIR_TC) {
+        return false;
+    }
+    *config = e.config;
+    return true;
+}
+
+TcConfig tuned_fir_tc_config(int num_taps, long long n)
+{
+    TcConfig config;
+    if (tuned_fir_tc_entry(num_taps, n, &config)) {
+        return config;
     }
     // The resident-window form where it applies (one copy of each window, no scan slices).
     const int window = fir_tcw_tile_blocks(num_taps, n);

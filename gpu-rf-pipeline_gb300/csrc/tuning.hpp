@@ -11,6 +11,8 @@ int tuned_fir_impl(int num_taps, long long n);
 int tuned_fir_batch_impl(int num_taps, long long n);
 int tuned_fir_batch_launch_impl(int num_taps, long long n);
 TcConfig tuned_fir_tc_config(int num_taps, long long n);
+// Whether a tuned entry names the tensor-core form for this case, and its configuration.
+bool tuned_fir_tc_entry(int num_taps, long long n, TcConfig* config);
 // *fused: the plan's calls of any length that the fused FP32 kernel takes run it (64 channels, no tuned
 // entry for the tensor-core form). The result then says what becomes of the others: RFX_CHAN_TC, no
 // tuned entry, refused as the tensor-core form's plans refuse them; RFX_CHAN_PLAIN, tuned, the plain form.

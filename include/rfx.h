@@ -144,8 +144,12 @@ int rfx_fir_launch_format(int impl, int format, const void* x, const float* taps
  * Replaces fir_load_const_taps (src/device_ops.hpp:87). */
 int rfx_fir_load_const_taps(const float* taps, int num_taps, cudaStream_t stream);
 
-/* `count` channels sharing one set of taps, in one launch; `x`, `y` and `num_samples` are HOST
- * arrays of `count` entries (device pointers / lengths). No limit of 8 channels.
+/* `count` channels sharing one set of taps, in as few launches as they allow (one for 64 channels;
+ * channels that read or overwrite what others write, or that a tuned table gives different kernels,
+ * take more); `x`, `y` and `num_samples` are HOST arrays of `count` entries (device pointers /
+ * lengths). No limit of 8 channels. With the plain kernel a channel has the bits of a call of its own;
+ * on the tensor cores its rounding may follow the others, whose lengths the tile is chosen by too
+ * (unless a tuned entry names the tile).
  * Replaces fir_batched_device (src/device_ops.hpp:99-100). */
 int rfx_fir_batched_device(int impl, const void* const* x, void* const* y,
                            const int64_t* num_samples, int count, const float* taps,
