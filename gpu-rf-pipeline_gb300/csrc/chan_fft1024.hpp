@@ -9,10 +9,10 @@ namespace rfx {
 cudaError_t chan_fft1024_launch(const void* u, void* out, long long frames, bool magnitude,
                                 cudaStream_t stream);
 
-// Longest call whose complex output this kernel transforms; longer ones use cuFFT's plan. Measured,
-// sums and transform, 32 taps per branch (us, this kernel / cuFFT): 44 frames 8.4 / 9.8, 4096 frames
-// 32.5 / 37.1, 16384 frames 99.0 / 102.6, 65536 frames 361 / 355. Magnitudes always use this kernel:
-// it writes them directly (65536 frames 337 against 478 with a magnitude pass).
+// Longest plan this kernel transforms; longer ones use cuFFT's plan. Measured, sums and transform, 32
+// taps per branch (us, this kernel / cuFFT): 44 frames 8.4 / 9.8, 4096 frames 32.5 / 37.1, 16384 frames
+// 99.0 / 102.6, 65536 frames 361 / 355. Magnitudes go the way of the complex outputs, whose bits they
+// have (65536 frames 469 with cuFFT and a magnitude pass; this kernel, which writes them directly, 329).
 constexpr long long kFft1024Frames = 8192;
 
 }  // namespace rfx

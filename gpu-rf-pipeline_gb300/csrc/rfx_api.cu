@@ -701,9 +701,12 @@ int rfx_magnitude_launch(const void* x, float* mag, int64_t num_samples, cudaStr
 
 namespace {
 
-// The channelizer through a plan; with `magnitude`, `out` receives |z| (float per channel):
-// the tensor-core form computes it in its epilogue, the plain form runs the magnitude kernel
-// over the channel outputs in the plan's scratch buffer (allocated by the first such call).
+// The channelizer through a plan; with `magnitude`, `out` receives |z| (float per channel), the bits of
+// the magnitude kernel over the call's complex outputs: the tensor-core forms, the plain form's fused
+// kernel and its 1024-point transform compute it in their last step, and where cuFFT transforms, the
+// magnitude kernel follows. What lies between two kernels (the channel outputs before cuFFT's magnitudes,
+// the branch sums before the 1024-point transform's) is in the plan's scratch buffer, allocated by the
+// first such call.
 int channelize_plan(rfx_chan_plan* plan, const void* x, const float* taps, void* out,
                     int64_t num_samples, int num_taps, cudaStream_t stream, bool magnitude,
                     int format)
@@ -780,7 +783,7 @@ int channelize_plan(rfx_chan_plan* plan, const void* x, const float* taps, void*
         }
         z = plan->scratch;
     }
-    if (plan->channels == 1024 && (magnitude || !plan->has_fft)) {
+    if (plan->channels == 1024 && !plan->has_fft) {
         cudaError_t err =
             rfx::chan_branch_launch(x, taps, z, frames, plan->channels, num_taps, stream, format);
         if (err == cudaSuccess) {

@@ -62,8 +62,8 @@ typedef enum rfx_chan_impl {
     /* FP32 branch sums (bit-identical to the project's channelize_branch_kernel) and the inverse
      * transform in FP32: one fused kernel for 8, 16, ..., 512 channels and at most 32 taps per
      * branch; otherwise a branch-sum kernel followed by this library's 1024-point transform
-     * (1024 channels: calls of at most 8192 frames, and magnitudes) or cuFFT's batched in-place
-     * inverse transform, as the project computes it. */
+     * (1024 channels, plans of at most 8192 frames) or cuFFT's batched in-place inverse
+     * transform, as the project computes it. */
     RFX_CHAN_PLAIN = 0,
     /* The M-point DFT as a split-FP16 complex GEMM on tcgen05. M = 64: one fused kernel (FP32
      * branch sums into shared memory, then the GEMM). M = 1024: the plain form's FP32 branch
@@ -228,11 +228,10 @@ int rfx_channelize_branches(const void* x, const float* taps, void* u, int64_t n
                             int channels, int num_taps, cudaStream_t stream);
 
 /* The channelizer followed by the magnitude of every channel output, mag[t][k] = |z[t][k]|
- * (frames x channels float32). Tensor-core plans compute it in the DFT-GEMM epilogue, so the
- * complex channel outputs never reach HBM, and so do the plain form's fused kernel and its
- * 1024-point transform (beyond 8192 frames equal to the magnitudes of rfx_channelize_launch's
- * outputs within FP32 rounding, otherwise bit for bit); other plain plans run the magnitude kernel
- * over the channel outputs. What lies between two kernels is in a plan-owned buffer, allocated by
+ * (frames x channels float32), bit for bit the magnitudes of rfx_channelize_launch's outputs.
+ * Tensor-core plans compute it in the DFT-GEMM epilogue, so the complex channel outputs never
+ * reach HBM, and so do the plain form's fused kernel and its 1024-point transform; plans that
+ * transform by cuFFT run the magnitude kernel over the channel outputs. What lies between two kernels is in a plan-owned buffer, allocated by
  * the first such call. mag 16-byte aligned. Fuses channelize |> magnitude (compiler/examples/channelizer.sf,
  * src/magnitude.cu:17-25); no single-call counterpart in the project. */
 int rfx_channelize_magnitude_launch(rfx_chan_plan* plan, const void* x, const float* taps,
