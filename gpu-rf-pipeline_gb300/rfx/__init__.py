@@ -130,13 +130,15 @@ _current_device = _raw_stream = None   # torch's, once the first launch has impo
 
 def _current_stream_ptr() -> int:
     """The handle of the current device's current stream, without building the Stream object of
-    torch.cuda.current_stream(): 0.2 us a call against 3.1, of 8.2 that a small launch took."""
+    torch.cuda.current_stream(): 0.2 us a call against 3.1, of 8.2 that a small launch took. (The
+    binding of torch that gives it is private: a torch without it gets the Stream object.)"""
     global _current_device, _raw_stream
     if _raw_stream is None:
         import torch
 
         _current_device = torch.cuda.current_device   # initializes CUDA if it is not yet
-        _raw_stream = torch._C._cuda_getCurrentRawStream
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda device: torch.cuda.current_stream(device).cuda_stream)
     return _raw_stream(_current_device())
 
 
