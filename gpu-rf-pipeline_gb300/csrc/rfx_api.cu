@@ -750,13 +750,21 @@ int channelize_plan(rfx_chan_plan* plan, const void* x, const float* taps, void*
                                                           magnitude, format);
             return err == cudaSuccess ? RFX_OK : cuda_fail(err, "chan_wide_launch");
         }
+        if (plan->fused) {
+            // The limits of the tensor-core form, whose place the fused kernel took under auto.
+            if (num_taps > 32 * plan->channels) {
+                return fail(RFX_ERR_CAPACITY, "channelize: %d taps, plans of auto at %d channels take "
+                                              "up to %d (plain: any number)",
+                            num_taps, plan->channels, 32 * plan->channels);
+            }
+            return fail(RFX_ERR_CUDA, "channelize: %lld samples, plans of auto at %d channels take a "
+                                      "whole frame or more",
+                        static_cast<long long>(num_samples), plan->channels);
+        }
         if (!rfx::chan_tc_supported(plan->channels, num_taps)) {
             return fail(RFX_ERR_CAPACITY, "channelize: %d taps exceed the tensor-core form's "
                                           "shared memory",
                         num_taps);
-        }
-        if (plan->fused) {
-            return cuda_fail(cudaErrorInvalidValue, "chan_fused_launch");   // less than a frame
         }
         const cudaError_t err = rfx::chan_tc_launch(x, taps, plan->twiddles, out, num_samples,
                                                     num_taps, stream, magnitude, format);
