@@ -997,7 +997,7 @@ __host__ __device__ constexpr int win_stages(int) { return 8; }
 __host__ __device__ constexpr int win_strips(int C) { return C == 1 ? 2 : 1; }
 
 // One window phase: the block's items of the captures that reach back C blocks.
-template <int C>
+template <int C, bool kTmemTaps>
 __device__ __forceinline__ void batch_window_items(const BatchView& v, unsigned char* smem,
                                                    uint32_t tmem)
 {
@@ -1011,15 +1011,15 @@ __device__ __forceinline__ void batch_window_items(const BatchView& v, unsigned 
     }
     const tcw::TcwListSrc src{v.wcap[C - 1], v.wmap[C - 1], v.wcount[C - 1], w0, w1 - w0};
     tcw::Ctrl& wctl = *reinterpret_cast<tcw::Ctrl*>(smem + v.win_ctl);
-    tcw::tcw_pipeline<C, 0, win_stages(C), tcw::TcwListSrc, win_strips(C)>(src, smem, wctl, tmem,
-                                                                        &g_fault_fir_batch);
+    tcw::tcw_pipeline<C, 0, win_stages(C), tcw::TcwListSrc, win_strips(C), tcw::kNB, kTmemTaps>(
+        src, smem, wctl, tmem, &g_fault_fir_batch);
     if (threadIdx.x == 0) {
         tcw::tcw_release<win_stages(C)>(wctl);
     }
     __syncthreads();
 }
 
-template <int S>
+template <int S, bool kTmemTaps = true>
 __device__ __forceinline__ void batch_body(const BatchView& v, unsigned char* smem)
 {
     static_assert(kThreads >= tcw::kThreads, "the window pipeline's roles fit the block");
@@ -1040,9 +1040,9 @@ __device__ __forceinline__ void batch_body(const BatchView& v, unsigned char* sm
     if (my_items > 0) {
         batch_tc_items<S>(v, first_item, my_items, smem, tmem);
     }
-    batch_window_items<1>(v, smem, tmem);
-    batch_window_items<2>(v, smem, tmem);
-    batch_window_items<3>(v, smem, tmem);
+    batch_window_items<1, kTmemTaps>(v, smem, tmem);
+    batch_window_items<2, kTmemTaps>(v, smem, tmem);
+    batch_window_items<3, kTmemTaps>(v, smem, tmem);
     if (v.plain_groups > 0) {
         const int t0 = v.cta_plain[blockIdx.x];
         const int t1 = v.cta_plain[blockIdx.x + 1];
@@ -1071,12 +1071,12 @@ fir_batch_kernel(const __grid_constant__ BatchParams p)
 }
 
 // A batch plan: the work list in device memory, tensor-core and plain captures in one launch.
-template <int S>
+template <int S, bool kTmemTaps = true>
 __global__ void __launch_bounds__(kThreads, 1)
 fir_batch_list_kernel(const __grid_constant__ BatchView v)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
-    batch_body<S>(v, smem);
+    batch_body<S, kTmemTaps>(v, smem);
 }
 
 namespace {
@@ -1313,6 +1313,7 @@ struct BatchPlan {
     BatchView view{};
     int grid = 0;
     int stages = 0;
+    void (*kernel)(BatchView) = nullptr;
     uint32_t smem = 0;
     int tc_caps = 0;
     int plain_caps = 0;
@@ -1615,10 +1616,14 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
         v.wcount[ci] = static_cast<int>(wc[ci].size());
     }
     v.win_ctl = plan->smem - 1024u;
-    const void* fn = plan->stages == 6   ? reinterpret_cast<const void*>(fir_batch_list_kernel<6>)
-                     : plan->stages == 4 ? reinterpret_cast<const void*>(fir_batch_list_kernel<4>)
-                                         : reinterpret_cast<const void*>(fir_batch_list_kernel<2>);
-    if ((err = opt_in_smem(fn, plan->smem)) != cudaSuccess) {
+    // Plans of no more tiles than blocks, none of them a long filter's, keep the tap matrices in shared
+    // memory: a block's one tile is over before the copy to tensor memory is paid back (one tile of 300
+    // taps 13.0 us against 13.6, of 63 taps 9.2 against 9.5).
+    plan->kernel = plan->stages == 6           ? fir_batch_list_kernel<6>
+                   : plan->stages == 4         ? fir_batch_list_kernel<4>
+                   : tc.empty() && units <= most ? fir_batch_list_kernel<2, false>
+                                               : fir_batch_list_kernel<2>;
+    if ((err = opt_in_smem(plan->kernel, plan->smem)) != cudaSuccess) {
         fir_batch_plan_free(plan);
         return err;
     }
@@ -1634,17 +1639,7 @@ cudaError_t fir_batch_plan_run(const BatchPlan* plan, cudaStream_t stream)
     const dim3 grid(static_cast<unsigned>(plan->grid));
     // Launched the ordinary way: overlapped with the end of the run before it (launch.hpp), runs
     // back to back took 1281 us each against 888 (256 captures), one alone no longer than before.
-    switch (plan->stages) {
-    case 6:
-        fir_batch_list_kernel<6><<<grid, kThreads, plan->smem, stream>>>(plan->view);
-        break;
-    case 4:
-        fir_batch_list_kernel<4><<<grid, kThreads, plan->smem, stream>>>(plan->view);
-        break;
-    default:
-        fir_batch_list_kernel<2><<<grid, kThreads, plan->smem, stream>>>(plan->view);
-        break;
-    }
+    plan->kernel<<<grid, kThreads, plan->smem, stream>>>(plan->view);
     return cudaGetLastError();
 }
 

@@ -302,8 +302,8 @@ __device__ __forceinline__ void tcw_init(Ctrl& ctl)
 // warps beyond the roles return at the final barrier) and returns after a block barrier.
 // With a list of captures (kMulti) the caller invalidates the control block's barriers before
 // the memory is used for anything else (tcw_release).
-// NB: blocks per tile (a multiple of eight).
-template <int C, int kFmt, int S, class Src, int kStrips = 2, int NB = kNB>
+// NB: blocks per tile (a multiple of eight). kTmemTaps: tap matrices in tensor memory, where that pays.
+template <int C, int kFmt, int S, class Src, int kStrips = 2, int NB = kNB, bool kTmemTaps = true>
 __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem, Ctrl& ctl,
                                              uint32_t tmem, unsigned int* fault)
 {
@@ -318,7 +318,7 @@ __device__ __forceinline__ void tcw_pipeline(const Src& src, unsigned char* smem
     // K-steps take 64 columns per split, the high split's chunks first, then the low split's, as
     // far as the columns go. The other MMAs read the strip in shared memory.
     constexpr int kChunkCols = 8 * kSteps;
-    constexpr int kRoom = NB <= 16 && C <= 2
+    constexpr int kRoom = !kTmemTaps || (NB <= 16 && C <= 2)
                               ? 0
                               : static_cast<int>(kTmemCols - 4 * kN) / kChunkCols;
     constexpr int kHiChunks = kRoom < C + 1 ? kRoom : C + 1;
