@@ -1520,15 +1520,16 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
     // others (256: 803 -> 825).
     const int most = std::min({sms, kBatchCtas, units});
     std::vector<int> tiles[kPhases];
+    constexpr double kNear = 3e-4;    // bisected as near as this: some 20 and 12 steps
     double longest = 1.01 * all_us;   // fits one block
     double low = 0.0;
-    for (int step = 0; step < 40; ++step) {
+    for (int step = 0; step < 24 && longest - low > kNear * longest; ++step) {
         const double mid = 0.5 * (low + longest);
         (deal(runs, mid, mid, most, tiles) ? longest : low) = mid;
     }
     double rest = longest;
     low = 0.0;
-    for (int step = 0; step < 40; ++step) {
+    for (int step = 0; step < 24 && rest - low > kNear * rest; ++step) {
         const double mid = 0.5 * (low + rest);
         (deal(runs, longest, mid, most, tiles) ? rest : low) = mid;
     }
