@@ -1,7 +1,7 @@
 // Plain FP32 FIR kernels for sm_103a: one tile per block (fir_plain_tile.cuh holds the tile
 // function, its arithmetic and its staging), for one capture (cf32 or integer input) and for
-// captures sharing one tap set in tiles of 384 to 1792 outputs by the amount of work (tile_shape),
-// and for captures with their own taps in tiles of 2304.
+// captures sharing one tap set in tiles of 384 to 2304 outputs by the amount of work and the filter's
+// shared memory (tile_shape), and for captures with their own taps in tiles of 2304.
 #include "fir_plain.cuh"
 #include "fir_plain_tile.cuh"
 #include "launch.hpp"

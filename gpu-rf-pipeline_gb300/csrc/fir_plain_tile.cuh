@@ -4,8 +4,8 @@
 //
 //   y[n] = sum_{k=0}^{K-1} h[k] x[n-k],  x[m] = 0 for m < 0,  n < N      (src/fir.cu:1-5)
 //
-// Written for R outputs per thread and T threads; described at R = 9 and T = 256, what large
-// inputs run (fir_plain.cu has the rule).
+// Written for R outputs per thread and T threads (fir_plain.cu has the rule); described at R = 9 and
+// T = 256, what batch plans, captures with their own taps and the longest filters run.
 //
 // Arithmetic: every output is one chain of fused multiply-adds over k = 0, 1, ..., K-1 starting
 // from +0.0f, separately for I and Q. That is the order of the project's naive, tiled and

@@ -240,10 +240,12 @@ double best_ms(Run run)
 
 // Built-in rule before tuning: the tensor-core form once the filter is long enough for FP32
 // FMA throughput to bound the plain kernel and the input fills the GPU; the plain kernel
-// otherwise. Measured on GB300 at 2^24 samples: the plain kernel is HBM-bound up to about 24
-// taps (42-49 us) and FMA-bound beyond (79 us at 63 taps, 149 us at 129); the resident-window
-// tensor-core form takes 48-58 us from 2 to 129 taps, 68 us at 255 and 82 us at 385; the
-// long-filter form 120 us at 511 taps and 141 us at 1025.
+// otherwise. Measured on GB300 at 2^24 samples (CUDA-graph replay): the plain kernel is HBM-bound up to
+// about 24 taps (39-42 us), meets the tensor-core form at 32 (45 us both) and is FMA-bound beyond (76 us at
+// 63 taps, 146 at 129); the resident-window tensor-core form takes 45-47 us from 2 to 129 taps, 59 at 255,
+// 72 at 385 and 102 at 511; the long-filter form 139 at 1025. 2^16 samples, plain against tensor core: 2.6
+// and 4.6 us at 63 taps, 6.8 and 7.3 at 511, 11.6 and 9.7 at 1025 (the line in samples was drawn when
+// both took longer there; short calls of short filters are faster under `plain`).
 int tuned_fir_impl(int num_taps, long long n)
 {
     FirEntry e;
@@ -278,8 +280,8 @@ int tuned_fir_batch_launch_impl(int num_taps, long long n)
 // that one takes (its window phase up to 385 taps, its long-filter phase beyond), at any length:
 // a plan launches once for the whole batch, so a short capture is no reason for the plain tiles.
 // Measured on the 256-capture workload (batch plans of each tap count alone): a window tile of
-// 6144 outputs costs 2.9-3.6 SM-us at 31-127 taps, 4.1 at 255, a long-filter tile of 12288
-// outputs 16.5-18.6 SM-us at 511-1025, against 2304-output plain tiles of 1.7 SM-us at 31 taps
+// 6144 outputs costs 2.1-2.2 SM-us at 31-127 taps, 2.8 at 255, a long-filter tile of 12288
+// outputs 14.8-16.5 SM-us at 511-1025, against 2304-output plain tiles of 1.7 SM-us at 31 taps
 // and 12.6-24.7 at 511-1025 (per output the tensor-core tiles cost less at every tap count);
 // putting the short captures of long filters on the plain tiles instead made the whole batch
 // 4 % slower.
