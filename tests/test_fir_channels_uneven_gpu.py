@@ -60,3 +60,13 @@ def test_short_channels_beside_a_long_one_cost_little(k: int) -> None:
              micros(lambda: rfx.fir_batched(xs[1:], ys[1:], h, "plain")))
     # A grid of the longest channel's tiles for every channel took five times the calls apart.
     assert both <= 2.0 * apart
+
+
+# Channels of about the same length take a row of blocks each: both sides of the line (one block in nine
+# without work), a tile more or less in a row, an empty row, more than one launch.
+@pytest.mark.parametrize("k", [1, 31, 700, 6000])
+@pytest.mark.parametrize("lengths", [
+    [384, 384], [20000] * 9 + [20001], [1152 * 8] * 8 + [1], [1152 * 8] * 9 + [0], [9000, 8999, 8001, 7000],
+    [40000 + 700 * i for i in range(5)], [5000 + (i % 3) for i in range(130)]])
+def test_rows_keep_the_bits(k: int, lengths: list[int]) -> None:
+    test_every_channel_keeps_its_bits(lengths, k)
