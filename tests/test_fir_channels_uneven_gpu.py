@@ -69,4 +69,4 @@ def test_short_channels_beside_a_long_one_cost_little(k: int) -> None:
     [384, 384], [20000] * 9 + [20001], [1152 * 8] * 8 + [1], [1152 * 8] * 9 + [0], [9000, 8999, 8001, 7000],
     [40000 + 700 * i for i in range(5)], [5000 + (i % 3) for i in range(130)]])
 def test_rows_keep_the_bits(k: int, lengths: list[int]) -> None:
-    test_every_channel_keeps_its_bits(lengths, k)
+    test_every_channel_keeps_its_bits(k, lengths)
