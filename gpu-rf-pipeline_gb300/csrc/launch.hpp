@@ -5,7 +5,7 @@
 // wait in wait_for_stream() (ptx.cuh) until every earlier kernel has completed and its writes are
 // visible. Every thread of such a kernel calls wait_for_stream() before it touches global memory
 // and allow_next() after it (a kernel that allocates tensor memory has a block barrier behind the
-// allocation and before both). A kernel launched in the ordinary way, a copy or an event after it
+// allocation and before both), or never where the kernel after it is better held back (chan_wide.cu). A kernel launched in the ordinary way, a copy or an event after it
 // still waits for its completion. Back to back on one stream this took 2 to 3 us off every call
 // (64 channels, 2^24 samples: 53.8 -> 51.5 us; 2^21 ci16 samples to magnitudes: 14.0 -> 10.9).
 #pragma once

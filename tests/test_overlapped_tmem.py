@@ -28,7 +28,7 @@ def allocations() -> list[tuple[str, str]]:
 
 def test_block_barrier_between_allocation_and_next_kernel() -> None:
     found = allocations()
-    assert {"chan_wide.cu", "chan_tc.cu", "fir_tc.cu"} <= {name for name, _ in found}
+    assert {"chan_tc.cu", "fir_tc.cu"} <= {name for name, _ in found}
     for name, code in found:
         assert "__syncthreads();" in code, name
         assert code.index("__syncthreads();") < code.index("wait_for_stream();"), name
