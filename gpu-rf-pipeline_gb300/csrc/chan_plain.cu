@@ -493,7 +493,7 @@ static RingKernel ring_kernel(int groups, Ring ring)
 
 static cudaError_t ring_launch(const void* x, const float* taps, float2* u, long long n,
                                long long frames, int channels, int num_taps, cudaStream_t stream,
-                               int format)
+                               int format, bool before_dft)
 {
     const int groups = static_cast<int>((num_taps + static_cast<long long>(kR) * channels - 1) /
                                         (static_cast<long long>(kR) * channels));
@@ -526,9 +526,14 @@ static cudaError_t ring_launch(const void* x, const float* taps, float2* u, long
     const int guard_frames = kR * (groups + 1);
     // Few channels reach long segments' form sooner: its tested first frames are in the caches there
     // (3 channels, 24 taps per branch, segments of 192 frames 26.1 us against 29.0 for kUniform, 64
-    // frames 12.1 against 11.6; 1024 channels, 192 frames 41 against 34).
-    const long long long_segment =
-        channels < 128 ? (groups == 4 ? 128 : 96) : (groups == 4 ? 160 : 256);
+    // frames 12.1 against 11.6; 1024 channels, 192 frames 41 against 34). So does the largest form before
+    // the tensor-core transform (1024 channels, 32 taps per branch, whole call: segments of 40 frames 31.5
+    // against 33.5, 72 47.7 against 54.5, 32 27.9 against 26.2; at 24 taps kUniform is faster at 72, 36.4
+    // against 41.1).
+    const long long long_segment = channels < 128                ? (groups == 4 ? 128 : 96)
+                                   : groups == 4 && before_dft ? 40
+                                   : groups == 4               ? 160
+                                                               : 256;
     const Ring ring = num_taps != kR * groups * channels ? Ring::kAny
                       : seg_frames < long_segment        ? Ring::kUniform
                                                          : Ring::kLong;
@@ -541,7 +546,8 @@ static cudaError_t ring_launch(const void* x, const float* taps, float2* u, long
 }
 
 cudaError_t chan_branch_launch(const void* x, const float* taps, void* u, long long frames,
-                               int channels, int num_taps, cudaStream_t stream, int format)
+                               int channels, int num_taps, cudaStream_t stream, int format,
+                               bool before_dft)
 {
     if (frames == 0 || channels < 1) {
         return cudaSuccess;
@@ -552,7 +558,7 @@ cudaError_t chan_branch_launch(const void* x, const float* taps, void* u, long l
         // in the one below.)
         if (num_taps <= 4LL * kR * channels && channels <= 65535LL * kRingThreads) {
             return ring_launch(x, taps, static_cast<float2*>(u), n, frames, channels, num_taps,
-                               stream, format);
+                               stream, format, before_dft);
         }
     }
     // The newest sample any frame reads is the last frame's x[(frames - 1) M], which lies in the

@@ -474,7 +474,7 @@ cudaError_t chan_wide_launch(const void* x, const float* taps, const void* image
     if (frames == 0) {
         return cudaSuccess;
     }
-    cudaError_t err = chan_branch_launch(x, taps, u, frames, kM, num_taps, stream, format);
+    cudaError_t err = chan_branch_launch(x, taps, u, frames, kM, num_taps, stream, format, true);
     if (err != cudaSuccess) {
         return err;
     }

@@ -1,4 +1,6 @@
-"""The 1024-channel tensor-core channelizer called back to back: no longer a call than one alone."""
+"""The 1024-channel tensor-core channelizer called back to back: no longer a call than one alone, and the
+same bits on both sides of the length where the branch sums change their form (csrc/chan_plain.cu,
+ring_launch)."""
 from __future__ import annotations
 
 import pytest
@@ -34,3 +36,32 @@ def test_back_to_back_calls_take_no_longer_than_one_alone() -> None:
     # A chained call has the launch hidden, so it is the shorter one; 5 % for the runs' spread. (It was
     # 10 % longer.)
     assert chained <= 1.05 * alone, (alone, chained)
+
+
+@pytest.mark.parametrize("fmt", ["cf32", "ci16"])
+@pytest.mark.parametrize("per_branch", [24, 32])
+def test_bits_do_not_depend_on_the_length(fmt: str, per_branch: int) -> None:
+    # Blocks of 57 segments on 152 SMs: 1824 frames are segments of 32, 1825 of 40, 9121 of 168.
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(per_branch)
+    longest = 9121 * M
+    x = torch.randint(-30000, 30000, (2 * longest,), generator=gen, device="cuda", dtype=torch.int16)
+    if fmt == "cf32":
+        x = torch.view_as_complex((x.float() / 32768).reshape(-1, 2))
+    taps = torch.randn(per_branch * M, generator=gen, device="cuda") / 181
+
+    def call(frames: int) -> torch.Tensor:
+        z = torch.empty((frames, M), dtype=torch.complex64, device="cuda")
+        n = frames * M
+        with rfx.ChanPlan(M, n, "tc_split") as plan:
+            if fmt == "cf32":
+                plan.launch(x[:n], taps, z)
+            else:
+                plan.launch_format(fmt, x[:2 * n], taps, z)
+            torch.cuda.synchronize()
+        return z
+
+    want = call(9121)
+    for frames in (1, 4, 1823, 1824, 1825, 1828, 2281):
+        assert torch.equal(call(frames), want[:frames]), frames
+    assert rfx.device_fault() == 0
