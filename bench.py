@@ -442,8 +442,9 @@ class BatchArm(RoundGraphs):
 
 def chan_launches(channels: int, impl: str) -> int:
     """Kernel launches per channelizer step: plain = branch sums + cuFFT's inverse (counted as
-    one of ours); tensor core = one fused kernel at 64 channels, branch sums + DFT kernel at
-    1024; auto = the tensor-core form at 64 channels, plain otherwise."""
+    one of ours; the most it takes, its one-pass kernel for 8 to 512 channels is one launch);
+    tensor core = one fused kernel at 64 channels, branch sums + DFT kernel at 1024; auto = one
+    fused kernel at 64 channels, plain otherwise."""
     tc = impl == "tc_split" or (impl == "auto" and channels == 64)
     return 1 if tc and channels == 64 else 2
 

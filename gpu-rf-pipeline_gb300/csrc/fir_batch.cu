@@ -1515,9 +1515,9 @@ cudaError_t fir_batch_plan_make(int impl, const rfx_fir_capture* captures, int c
     // memory-bound work overlap. Calls back to back against equal shares of per-tile costs alone (us,
     // with the window tiles' tap matrices in tensor memory): 256 captures of up to 2^22 samples 890 -> 831
     // (808 to 820 by graph replay), 224 of up to 2^20 264 -> 224, 200 of up to 2^18 129 -> 108, 70 of up to
-    // 2^18 67 -> 46. By graph replay, letting each phase start over at the first block, to fill what the long-filter tiles leave there, was
-    // faster for some batches (64 of up to 2^21 134 -> 127, before the second limit) and slower for
-    // others (256: 803 -> 825).
+    // 2^18 67 -> 46. By graph replay, letting each phase start over at the first block, to fill what the
+    // long-filter tiles leave there, was faster for some batches (64 of up to 2^21 134 -> 127, before the
+    // second limit) and slower for others (256: 803 -> 825).
     const int most = std::min({sms, kBatchCtas, units});
     std::vector<int> tiles[kPhases];
     constexpr double kNear = 3e-4;    // bisected as near as this: some 20 and 12 steps

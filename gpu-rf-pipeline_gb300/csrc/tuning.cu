@@ -315,8 +315,8 @@ TcConfig tuned_fir_tc_config(int num_taps, long long n)
 }
 
 // Built-in rule: at 64 channels the fused FP32 kernel (chan_fused.cuh) where the tensor-core form
-// stood (a tuned plain entry is the same kernel); the plain form elsewhere, including 1024 channels, where the branch-sum kernel + cuFFT
-// measured faster than the factored tensor-core DFT on GB300.
+// stood (a tuned plain entry is the same kernel); the plain form elsewhere, including 1024 channels, where
+// the branch-sum kernel + cuFFT measured faster than the factored tensor-core DFT on GB300.
 int tuned_chan_impl(int channels, long long n, bool* fused)
 {
     ChanEntry e;

@@ -231,8 +231,8 @@ int rfx_channelize_branches(const void* x, const float* taps, void* u, int64_t n
  * (frames x channels float32), bit for bit the magnitudes of rfx_channelize_launch's outputs.
  * Tensor-core plans compute it in the DFT-GEMM epilogue, so the complex channel outputs never
  * reach HBM, and so do the plain form's fused kernel and its 1024-point transform; plans that
- * transform by cuFFT run the magnitude kernel over the channel outputs. What lies between two kernels is in a plan-owned buffer, allocated by
- * the first such call. mag 16-byte aligned. Fuses channelize |> magnitude (compiler/examples/channelizer.sf,
+ * transform by cuFFT run the magnitude kernel over the channel outputs. What lies between two
+ * kernels is in a plan-owned buffer, allocated by the first such call. mag 16-byte aligned. Fuses channelize |> magnitude (compiler/examples/channelizer.sf,
  * src/magnitude.cu:17-25); no single-call counterpart in the project. */
 int rfx_channelize_magnitude_launch(rfx_chan_plan* plan, const void* x, const float* taps,
                                     float* mag, int64_t num_samples, int num_taps,
